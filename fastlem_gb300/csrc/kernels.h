@@ -21,6 +21,7 @@ enum KClass {
     kcSkelDown,       // skeleton chains top-down (response time, elevation)
     kcLowDown,        // Kahn rounds top-down (response time, elevation)
     kcMisc,
+    kcResident,       // whole solves of resident terrains
     kcCount
 };
 
@@ -52,6 +53,7 @@ struct Tuning {
     int64_t kahn_min_width = -1;
     int sized_grids = -1;
     bool gpu_rank = true;
+    int resident = -1;     // whole solves in one launch: 0 never
 };
 Tuning& tuning();
 // The shapes for a model of n sites (packed: several terrains), overrides applied.
@@ -292,6 +294,55 @@ RankResult gpu_lake_rank(cudaStream_t st, uint32_t n, const uint32_t* row, const
 
 // Runs the exact parallel fold over one chain of n operands starting at x0 (probe).
 cudaError_t fold_probe(const double* y, uint32_t n, double x0, double* out);
+
+// ---- whole solves in one launch (resident.cu) ----
+constexpr uint32_t kResidentThreads = 1024;
+constexpr uint32_t kResidentEdges = 512;     // donors a block may have in other blocks
+constexpr size_t kResidentSmem = 226 * 1024; // shared memory of a block, at most
+constexpr uint32_t kResidentPart = 1024;     // sites of a block while there are blocks left
+constexpr uint32_t kResidentMaxRow = 64;     // longest adjacency row taken
+// A terrain's device sites [lo, lo + n), cut into `parts` block ranges; slot0: its first
+// (terrain, part) slot.
+struct ResidentTerrain {
+    uint32_t lo, n, parts, slot0;
+};
+// A terrain's progress, kept from launch to launch.
+struct ResidentCtrl {
+    uint32_t iters;        // iterations done
+    uint32_t done;         // settled, or at the limit
+    int error;             // kErr*
+    uint32_t need_rank;    // stopped: an iteration found lakes before the lake order was there
+};
+struct ResidentArgs {
+    uint32_t n, cap, slots, chunk;   // chunk: most iterations of a terrain per launch
+    uint32_t limit;
+    bool rank_ready;
+    const uint32_t *row, *col;
+    const double* len;
+    const float* ilen;
+    const double *area, *k, *u, *tanms;
+    const uint8_t* outlet;
+    const uint32_t *rank, *sor;
+    double* elev;
+    float2* pair;                    // the elevations as float pairs (slope.cuh)
+    uint32_t* next;
+    double *rlen, *w, *wa, *wl, *ef;
+    uint32_t *lab, *lab2, *root;
+    unsigned long long* best;
+    double *xch, *xch2;              // four values per site each
+    const ResidentTerrain* terrains;
+    const uint32_t* slot_terrain;
+    ResidentCtrl* ctrl;
+    unsigned long long* bars;        // four per terrain, zero at launch
+    uint32_t* ticket;                // zero at launch
+};
+size_t resident_smem(uint32_t cap);
+uint32_t resident_cap();             // most sites of a block
+uint32_t resident_blocks();
+cudaError_t launch_resident(const ResidentArgs& a, bool slope, uint32_t blocks, cudaStream_t st);
+// *bad = 1 unless the graph is simple (see resident.cu).
+void launch_check_simple(cudaStream_t st, uint32_t n, const uint32_t* row, const uint32_t* col,
+                         int* bad);
 
 // One drainage-area / response-time / elevation pass on final receivers.
 cudaError_t basin_pass(const BasinArgs& a, cudaStream_t st, const Hooks& hk, uint32_t nnz);

@@ -36,6 +36,7 @@
 #include "fastlem_gb300.h"
 #include "kernels.h"
 #include "rng.h"
+#include "slope.cuh"
 
 namespace fl {
 bool lake_heap_rank(uint32_t n, const uint32_t* row_ptr, const uint32_t* col, const double* len,
@@ -133,9 +134,13 @@ __global__ void k_noise(uint32_t n, double* __restrict__ noise) {
 // elev[j] = base[j] + noise[perm[j]] * f64::EPSILON (generator.rs:135-138), device order.
 __global__ void k_initial_elevation(uint32_t n, const uint32_t* __restrict__ perm,
                                     const double* __restrict__ base,
-                                    const double* __restrict__ noise, double* __restrict__ elev) {
+                                    const double* __restrict__ noise, double* __restrict__ elev,
+                                    float2* __restrict__ pair) {
     uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) elev[j] = __dadd_rn(base[j], __dmul_rn(noise[perm[j]], kEpsilon));
+    if (j >= n) return;
+    const double e = __dadd_rn(base[j], __dmul_rn(noise[perm[j]], kEpsilon));
+    elev[j] = e;
+    pair[j] = float_pair(e);
 }
 
 // dst[j] = src[idx[j]]: caller order <-> device order.
@@ -340,6 +345,7 @@ Tuning& tuning() {
         d.kahn_min_width = env("FL_KAHN_MIN_WIDTH", 256, 1l << 24, -1);
         d.gpu_rank = env("FL_GPU_RANK", 0, 1, 1) != 0;
         d.sized_grids = (int)env("FL_SIZED_GRIDS", 0, 1, -1);
+        d.resident = (int)env("FL_RESIDENT", 0, 1, -1);
         return d;
     }();
     return t;
@@ -381,7 +387,8 @@ Shape shape_for(uint32_t n, bool packed) {
 // ---------------------------------------------------------------------------
 const char* const kKClassName[kcCount] = {
     "initial_elevation", "receivers", "lake_reroute", "basin_build", "kahn_rounds",
-    "skeleton_rank", "skeleton_up", "response_w", "skeleton_down", "rounds_down", "misc"};
+    "skeleton_rank", "skeleton_up", "response_w", "skeleton_down", "rounds_down", "misc",
+    "resident_solve"};
 
 struct fl_graph {
     uint32_t n = 0;
@@ -424,6 +431,7 @@ struct fl_graph {
     // model (device)
     uint32_t *d_row = nullptr, *d_col = nullptr;
     double *d_len = nullptr, *d_area = nullptr;
+    float2* d_pair = nullptr;  // elevations as float pairs (slope.cuh)
     float* d_ilen = nullptr;   // 1/len per slot in f32 (receiver slope estimates)
     // parameters and iteration state (device)
     double *d_k = nullptr, *d_u = nullptr, *d_tan = nullptr, *d_base = nullptr, *d_elev = nullptr,
@@ -462,6 +470,12 @@ struct fl_graph {
     uint32_t passes = 0;   // basin passes since the drainage areas were reset
     int stamp = 0;
     uint32_t last_meta[kMetaCount] = {};
+    // whole solves in one launch (resident.cu): the terrains' parts, in one device block
+    // of ticket, barrier words (zeroed per launch), progress, terrains and slots
+    bool resident = false;
+    uint32_t largest = 0;                // sites of the largest terrain
+    uint32_t res_cap = 0, res_slots = 0, res_blocks = 0;
+    unsigned char* d_resident = nullptr;
     // instrumentation: launches / algorithmic bytes always, device time when enabled
     bool timing = false;
     uint64_t k_launches[kcCount] = {};
@@ -544,7 +558,8 @@ void free_graph(fl_graph* g) {
                     g->d_tokval, g->d_needl, g->d_push, g->d_rtime, g->d_kslot, g->d_cpar,
                     g->d_cqp, g->d_trec, g->d_noise_idx, g->d_tid, g->d_tchg, g->d_cdep,
                     g->d_cpar1, g->d_cdep1, g->d_chist, g->d_corder, g->d_tokslot, g->d_pend,
-                    g->d_corder_up, g->d_wa, g->d_wl, g->d_ilen, g->d_titer};
+                    g->d_corder_up, g->d_wa, g->d_wl, g->d_ilen, g->d_titer, g->d_resident,
+                    g->d_pair};
     for (void* p : ptrs)
         if (p) cudaFreeAsync(p, g->stream);
     status_block_put(g->h_status);
@@ -621,6 +636,7 @@ int alloc_workspace(fl_graph* g) {
     FL_TRY(dalloc(&g->d_tan, n));
     FL_TRY(dalloc(&g->d_base, n));
     FL_TRY(dalloc(&g->d_elev, n));
+    FL_TRY(dalloc(&g->d_pair, n));
     FL_TRY(dalloc(&g->d_A, n));
     FL_TRY(dalloc(&g->d_t, n));
     FL_TRY(dalloc(&g->d_w, n));
@@ -1363,6 +1379,196 @@ int upload_params(fl_graph* g, HostCols<const double> base, HostCols<const doubl
     return FL_OK;
 }
 
+// The end of generate(): the elevations back to the caller, iterations and times.
+int finish_generate(fl_graph* g, HostCols<double> out_elev, uint32_t iters, uint32_t* out_iters,
+                    double* loop_ms, double* total_ms, std::chrono::steady_clock::time_point t_start) {
+    FL_CU(cudaEventRecord(g->ev1, g->stream));
+    FL_TRY(download_permuted(g, g->d_elev, out_elev));
+    FL_CU(cudaStreamSynchronize(g->stream));
+    kresolve(g);
+    if (out_iters) *out_iters = iters;
+    if (loop_ms) {
+        float ms = 0;
+        FL_CU(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
+        *loop_ms = ms;
+    }
+    if (total_ms)
+        *total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
+    return FL_OK;
+}
+
+// ---- whole solves in one launch (resident.cu) ----
+
+// Offsets in fl_graph::d_resident for k terrains.
+struct ResidentLayout {
+    uint64_t ticket = 0, bars, ctrl, terrains, slots, bytes;
+    ResidentLayout(uint32_t k, uint32_t n_slots) {
+        bars = 64;
+        ctrl = bars + 32ull * k;
+        terrains = ctrl + sizeof(ResidentCtrl) * k;
+        slots = terrains + sizeof(ResidentTerrain) * k;
+        bytes = slots + 4ull * n_slots;
+    }
+};
+
+// Cuts the model's terrains into block parts and uploads the plan; leaves g->resident
+// false when some terrain is too large for the GPU's blocks or the graph is not simple.
+int plan_resident(fl_graph* g) {
+    g->resident = false;
+    const uint32_t sms = fl::resident_blocks();
+    for (uint32_t t = 0; t < g->terrains; ++t)
+        g->largest = std::max(g->largest, g->site_off[t + 1] - g->site_off[t]);
+    const uint32_t cap = fl::resident_cap();
+    if (g->largest > (uint64_t)sms * cap || g->n >= 0x80000000u) return FL_OK;
+    FL_CU(cudaMemsetAsync(g->d_flags, 0, sizeof(int), g->stream));
+    fl::launch_check_simple(g->stream, g->n, g->d_row, g->d_col, g->d_flags);
+    FL_CU(cudaGetLastError());
+    FL_CU(cudaMemcpyAsync(g->h_status, g->d_flags, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+    FL_CU(cudaStreamSynchronize(g->stream));
+    FL_CU(cudaMemsetAsync(g->d_flags, 0, sizeof(int), g->stream));
+    if (g->h_status[0] != 0) return FL_OK;
+    // sites per part
+    const uint64_t per = std::min<uint64_t>(cap, std::max<uint64_t>(kResidentPart, (g->n + sms - 1) / sms));
+    std::vector<ResidentTerrain> terr(g->terrains);
+    std::vector<uint32_t> by_size(g->terrains), slots;
+    for (uint32_t t = 0; t < g->terrains; ++t) {
+        const uint32_t m = g->site_off[t + 1] - g->site_off[t];
+        terr[t] = ResidentTerrain{g->site_off[t], m, std::min(sms, (uint32_t)((m + per - 1) / per)), 0};
+        by_size[t] = t;
+        g->res_cap = std::max(g->res_cap, (m + terr[t].parts - 1) / terr[t].parts);
+    }
+    std::stable_sort(by_size.begin(), by_size.end(), [&](uint32_t x, uint32_t y) { return terr[x].n > terr[y].n; });
+    for (uint32_t t : by_size) {
+        terr[t].slot0 = (uint32_t)slots.size();
+        slots.insert(slots.end(), terr[t].parts, t);
+    }
+    g->res_slots = (uint32_t)slots.size();
+    g->res_blocks = std::min(sms, g->res_slots);
+    const ResidentLayout lay(g->terrains, g->res_slots);
+    FL_TRY(dalloc(&g->d_resident, lay.bytes));
+    FL_CU(cudaMemcpyAsync(g->d_resident + lay.terrains, terr.data(), terr.size() * sizeof terr[0],
+                          cudaMemcpyHostToDevice, g->stream));
+    FL_CU(cudaMemcpyAsync(g->d_resident + lay.slots, slots.data(), slots.size() * 4ull,
+                          cudaMemcpyHostToDevice, g->stream));
+    FL_CU(cudaStreamSynchronize(g->stream));
+    g->resident = true;
+    return FL_OK;
+}
+
+// The largest terrain that the resident solve takes by default.  Its walks go site by site
+// (about 0.6 us a site of the longest river and direction), the staged pass folds whole
+// chains but pays some 400 us of launches, barriers and skeleton building an iteration.
+// Measured without slope limits (32 iterations, staged / resident, ms): 1,000 sites 4.7 /
+// 0.8, 16,000 12.2 / 5.1, 100,000 16.5 / 12.3, 150,000 17.9 / 17.6, 200,000 19.8 / 21.2.
+// With slope limits the staged walk is site by site too: 65,000 26.4 / 16.0, 400,000 53.5 /
+// 39.5, 600,000 102 / 88.
+constexpr uint32_t kResidentLargest = 131072, kResidentLargestSlope = 524288;
+
+// Whether generate() takes the resident solve: a tuning override of the staged pass's
+// shapes asks for that pass.
+bool use_resident(const fl_graph* g) {
+    const fl::Tuning& t = fl::tuning();
+    return g->resident && t.resident != 0 && t.low_ilp < 0 && t.walk_per_sm < 0 &&
+           t.kahn_min_width < 0 && t.sized_grids < 0 &&
+           (t.resident == 1 || g->largest <= (g->slope ? kResidentLargestSlope : kResidentLargest));
+}
+
+// The iterations of every terrain from the initial elevations in d_elev; *fell_back when
+// a block met more far donors than it has room for (the model then keeps to the staged
+// pass; d_elev is to be set up again).  iters[t]: iterations of terrain t.
+int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t limit,
+                   std::vector<uint32_t>& iters, bool* fell_back) {
+    const uint32_t k = g->terrains;
+    const ResidentLayout lay(k, g->res_slots);
+    unsigned char* d = g->d_resident;
+    FL_CU(cudaMemsetAsync(d + lay.ctrl, 0, sizeof(ResidentCtrl) * k, g->stream));
+    int h[kNumFlags];
+    if (!g->rank_uploaded) {                  // the first iteration's lakes
+        FL_TRY(clear_flags(g));
+        if (g->d_titer)
+            FL_CU(cudaMemsetAsync(g->d_titer, 0, g->terrains * sizeof(uint32_t), g->stream));
+        FL_TRY(enqueue_receivers(g));
+        FL_TRY(sync_status(g, h));
+        if (h[kHasLake]) FL_TRY(set_outlets(g, outlets, true));
+    }
+    ResidentArgs a{};
+    a.n = g->n;
+    a.cap = g->res_cap;
+    a.slots = g->res_slots;
+    // a launch ends after some tens of milliseconds, so that other streams' solves run
+    a.chunk = (uint32_t)std::max<uint64_t>(16, std::min<uint64_t>(1024, (1ull << 27) / std::max(1u, g->n)));
+    a.limit = (uint32_t)limit;
+    a.row = g->d_row;
+    a.col = g->d_col;
+    a.len = g->d_len;
+    a.ilen = g->d_ilen;
+    a.area = g->d_area;
+    a.k = g->d_k;
+    a.u = g->d_u;
+    a.tanms = g->d_tan;
+    a.outlet = g->d_outlet;
+    a.rank = g->d_rank;
+    a.sor = g->d_sor;
+    a.elev = g->d_elev;
+    a.pair = g->d_pair;
+    a.next = g->d_next;
+    a.rlen = g->d_rlen;
+    a.w = g->d_w;
+    a.wa = g->d_wa;
+    a.wl = g->d_wl;
+    a.lab = g->d_lab;
+    a.lab2 = g->d_lab2;
+    a.root = g->d_sid;
+    a.ef = g->d_t;
+    a.best = g->d_best;
+    a.xch = reinterpret_cast<double*>(g->d_trec);
+    a.xch2 = reinterpret_cast<double*>(g->d_rec);
+    a.terrains = reinterpret_cast<const ResidentTerrain*>(d + lay.terrains);
+    a.slot_terrain = reinterpret_cast<const uint32_t*>(d + lay.slots);
+    a.ctrl = reinterpret_cast<ResidentCtrl*>(d + lay.ctrl);
+    a.bars = reinterpret_cast<unsigned long long*>(d + lay.bars);
+    a.ticket = reinterpret_cast<uint32_t*>(d + lay.ticket);
+    g->w_valid = false;
+    std::vector<ResidentCtrl> ctrl(k);
+    bool more = true;
+    while (more) {
+        FL_CU(cudaMemsetAsync(d, 0, lay.ctrl, g->stream));
+        a.rank_ready = g->rank_uploaded;
+        cudaError_t e = cudaSuccess;
+        FL_LAUNCH(g, kcResident, 0.0, e = fl::launch_resident(a, g->slope, g->res_blocks, g->stream));
+        if (e != cudaSuccess) {
+            set_err("resident solve launch", e);
+            return FL_ERR_CUDA;
+        }
+        FL_CU(cudaMemcpyAsync(ctrl.data(), d + lay.ctrl, sizeof(ResidentCtrl) * k, cudaMemcpyDeviceToHost,
+                              g->stream));
+        FL_CU(cudaStreamSynchronize(g->stream));
+        g->host_syncs++;
+        more = false;
+        bool need_rank = false;
+        for (uint32_t t = 0; t < k; ++t) {
+            if (ctrl[t].error == kErrCapacity) {
+                *fell_back = true;
+                g->resident = false;
+                return FL_OK;
+            }
+            h[kError] = ctrl[t].error;
+            FL_TRY(device_error(h));
+            more |= !ctrl[t].done;
+            need_rank |= ctrl[t].need_rank != 0;
+            iters[t] = ctrl[t].iters;
+        }
+        if (need_rank) {
+            FL_TRY(set_outlets(g, outlets, true));
+            for (uint32_t t = 0; t < k; ++t) ctrl[t].need_rank = 0;
+            FL_CU(cudaMemcpyAsync(d + lay.ctrl, ctrl.data(), sizeof(ResidentCtrl) * k, cudaMemcpyHostToDevice,
+                                  g->stream));
+            FL_CU(cudaStreamSynchronize(g->stream));
+        }
+    }
+    return FL_OK;
+}
+
 int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
                   HostCols<const double> k, HostCols<const double> u,
                   HostCols<const uint8_t> is_outlet, HostCols<const double> max_slope,
@@ -1385,21 +1591,40 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
     // all status words, including the grid barrier's, start from zero
     FL_CU(cudaMemsetAsync(g->d_flags, 0, kNumFlags * sizeof(int), g->stream));
     // every terrain draws its own StdRng::seed_from_u64(0) stream, sample i for its site i
-    FL_LAUNCH(g, kcNoise, 8.0 * g->noise_n,
-              k_noise<<<blocks_for((g->noise_n + 7) / 8), kThreads, 0, g->stream>>>(g->noise_n, g->d_w));
-    g->w_valid = false;
-    FL_LAUNCH(g, kcNoise, 28.0 * n,
-              k_initial_elevation<<<blocks_for(n), kThreads, 0, g->stream>>>(
-                  n, g->d_noise_idx ? g->d_noise_idx : g->d_perm, g->d_base, g->d_w, g->d_elev));
+    auto initial_elevations = [&]() -> int {
+        FL_LAUNCH(g, kcNoise, 8.0 * g->noise_n,
+                  k_noise<<<blocks_for((g->noise_n + 7) / 8), kThreads, 0, g->stream>>>(g->noise_n, g->d_w));
+        g->w_valid = false;
+        FL_LAUNCH(g, kcNoise, 28.0 * n,
+                  k_initial_elevation<<<blocks_for(n), kThreads, 0, g->stream>>>(
+                      n, g->d_noise_idx ? g->d_noise_idx : g->d_perm, g->d_base, g->d_w, g->d_elev, g->d_pair));
+        FL_CU(cudaGetLastError());
+        return FL_OK;
+    };
+    FL_TRY(initial_elevations());
+    if (max_iter > 0xffffffffll) max_iter = 0xffffffffll;
+    uint64_t limit = max_iter < 0 ? 0xffffffffull : (uint64_t)max_iter;
+    uint32_t iters = 0;
+    if (limit > 0 && use_resident(g)) {
+        FL_CU(cudaEventRecord(g->ev0, g->stream));
+        std::vector<uint32_t> each(g->terrains);
+        bool fell_back = false;
+        FL_TRY(resident_solve(g, outlets, limit, each, &fell_back));
+        if (!fell_back) {
+            for (uint32_t t = 0; t < g->terrains; ++t) {
+                iters = std::max(iters, each[t]);
+                if (terrain_iters) terrain_iters[t] = each[t];
+            }
+            return finish_generate(g, out_elev, iters, out_iters, loop_ms, total_ms, t_start);
+        }
+        FL_TRY(initial_elevations());
+    }
     // previous-iteration drainage areas steer the skeleton's chain choice; start from
     // the cell areas
     FL_LAUNCH(g, kcMisc, 16.0 * n,
               k_fill_f64<<<blocks_for(n), kThreads, 0, g->stream>>>(n, g->d_A, g->d_area));
     FL_CU(cudaGetLastError());
     FL_CU(cudaEventRecord(g->ev0, g->stream));
-    if (max_iter > 0xffffffffll) max_iter = 0xffffffffll;
-    uint64_t limit = max_iter < 0 ? 0xffffffffull : (uint64_t)max_iter;
-    uint32_t iters = 0;
     g->passes = 0;
     // a terrain alone stops at its first iteration without a change; packed with others
     // it keeps iterating at a fixed point, so its count is that first unchanged iteration
@@ -1471,19 +1696,7 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
             terrain_iters[0] = iters;
         }
     }
-    FL_CU(cudaEventRecord(g->ev1, g->stream));
-    FL_TRY(download_permuted(g, g->d_elev, out_elev));
-    FL_CU(cudaStreamSynchronize(g->stream));
-    kresolve(g);
-    if (out_iters) *out_iters = iters;
-    if (loop_ms) {
-        float ms = 0;
-        FL_CU(cudaEventElapsedTime(&ms, g->ev0, g->ev1));
-        *loop_ms = ms;
-    }
-    if (total_ms)
-        *total_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t_start).count();
-    return FL_OK;
+    return finish_generate(g, out_elev, iters, out_iters, loop_ms, total_ms, t_start);
 }
 
 }  // namespace
@@ -1625,6 +1838,7 @@ int create_graph(uint32_t n, const uint32_t* row_ptr, const uint32_t* col, const
     }
     g->def_outlets.resize(n_default);
     for (uint32_t i = 0; i < n_default; ++i) g->def_outlets[i] = g->inv[default_outlets[i]];
+    if ((rc = plan_resident(g))) return fail(rc);
     *out = g;
     return FL_OK;
 }
@@ -1910,6 +2124,8 @@ int fl_set_tuning(const char* name, int64_t value) {
         t.walk_per_sm = (int)value;
     } else if (k == "sized_grids" && value >= -1 && value <= 1) {
         t.sized_grids = (int)value;
+    } else if (k == "resident" && value >= -1 && value <= 1) {
+        t.resident = (int)value;
     } else if (k == "gpu_rank" && (value == 0 || value == 1)) {
         t.gpu_rank = value != 0;
     } else if (k == "kahn_min_width" &&
@@ -1930,6 +2146,7 @@ int64_t fl_get_tuning(const char* name) {
     if (k == "kahn_min_width") return t.kahn_min_width;
     if (k == "gpu_rank") return t.gpu_rank ? 1 : 0;
     if (k == "sized_grids") return t.sized_grids;
+    if (k == "resident") return t.resident;
     return -2;
 }
 
