@@ -296,10 +296,12 @@ RankResult gpu_lake_rank(cudaStream_t st, uint32_t n, const uint32_t* row, const
 cudaError_t fold_probe(const double* y, uint32_t n, double x0, double* out);
 
 // ---- whole solves in one launch (resident.cu) ----
-constexpr uint32_t kResidentThreads = 1024;
 constexpr uint32_t kResidentEdges = 512;     // donors a block may have in other blocks
 constexpr size_t kResidentSmem = 226 * 1024; // shared memory of a block, at most
-constexpr uint32_t kResidentPart = 1024;     // sites of a block while there are blocks left
+// Sites of a block while there are blocks left.  us an iteration at 1,000 / 10,000 / 65,537
+// sites: 224 29.9 / 59.5 / 125, 448 29.2 / 60.0 / 120, 896 33.4 / 63.3 / 124, 1,792 34.1 /
+// 87.4 / 170.
+constexpr uint32_t kResidentPart = 448;
 constexpr uint32_t kResidentMaxRow = 64;     // longest adjacency row taken
 // A terrain's device sites [lo, lo + n), cut into `parts` block ranges; slot0: its first
 // (terrain, part) slot.
@@ -312,10 +314,13 @@ struct ResidentCtrl {
     uint32_t done;         // settled, or at the limit
     int error;             // kErr*
     uint32_t need_rank;    // stopped: an iteration found lakes before the lake order was there
+    uint32_t slow;         // stopped: iterations over the time limit
+    uint32_t pad[3];
 };
 struct ResidentArgs {
     uint32_t n, cap, slots, chunk;   // chunk: most iterations of a terrain per launch
     uint32_t limit;
+    uint64_t slow_ns;                // stop after four iterations in a row over this; 0: never
     bool rank_ready;
     const uint32_t *row, *col;
     const double* len;
@@ -326,19 +331,20 @@ struct ResidentArgs {
     double* elev;
     float2* pair;                    // the elevations as float pairs (slope.cuh)
     uint32_t* next;
-    double *rlen, *w, *wa, *wl, *ef;
-    uint32_t *lab, *lab2, *root;
+    double *rlen, *w, *wa, *wl;
+    uint32_t *lab, *lab2;
     unsigned long long* best;
-    double *xch, *xch2;              // four values per site each
+    double *xarea, *xtime, *xelev;   // exchange slots: two, four and two values per site
+    double* troot;
     const ResidentTerrain* terrains;
     const uint32_t* slot_terrain;
     ResidentCtrl* ctrl;
     unsigned long long* bars;        // four per terrain, zero at launch
     uint32_t* ticket;                // zero at launch
 };
-size_t resident_smem(uint32_t cap);
-uint32_t resident_cap();             // most sites of a block
-uint32_t resident_blocks();
+size_t resident_smem(uint32_t cap, bool slope);
+uint32_t resident_cap(bool slope);   // most sites of a block
+uint32_t resident_blocks();          // most blocks of a launch
 cudaError_t launch_resident(const ResidentArgs& a, bool slope, uint32_t blocks, cudaStream_t st);
 // *bad = 1 unless the graph is simple (see resident.cu).
 void launch_check_simple(cudaStream_t st, uint32_t n, const uint32_t* row, const uint32_t* col,

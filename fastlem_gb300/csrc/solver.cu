@@ -473,6 +473,7 @@ struct fl_graph {
     // whole solves in one launch (resident.cu): the terrains' parts, in one device block
     // of ticket, barrier words (zeroed per launch), progress, terrains and slots
     bool resident = false;
+    bool res_slope = false;              // the plan has room for slope limits
     uint32_t largest = 0;                // sites of the largest terrain
     uint32_t res_cap = 0, res_slots = 0, res_blocks = 0;
     unsigned char* d_resident = nullptr;
@@ -1411,29 +1412,38 @@ struct ResidentLayout {
     }
 };
 
-// Cuts the model's terrains into block parts and uploads the plan; leaves g->resident
-// false when some terrain is too large for the GPU's blocks or the graph is not simple.
-int plan_resident(fl_graph* g) {
-    g->resident = false;
-    const uint32_t sms = fl::resident_blocks();
+// Whether every terrain's graph is one the resident solve takes (at set-up; the model's
+// buffers are ready).
+int check_resident(fl_graph* g) {
     for (uint32_t t = 0; t < g->terrains; ++t)
         g->largest = std::max(g->largest, g->site_off[t + 1] - g->site_off[t]);
-    const uint32_t cap = fl::resident_cap();
-    if (g->largest > (uint64_t)sms * cap || g->n >= 0x80000000u) return FL_OK;
+    g->resident = g->largest <= (uint64_t)fl::resident_blocks() * fl::resident_cap(false) &&
+                  g->n < 0x80000000u;
+    if (!g->resident) return FL_OK;
     FL_CU(cudaMemsetAsync(g->d_flags, 0, sizeof(int), g->stream));
     fl::launch_check_simple(g->stream, g->n, g->d_row, g->d_col, g->d_flags);
     FL_CU(cudaGetLastError());
     FL_CU(cudaMemcpyAsync(g->h_status, g->d_flags, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
-    FL_CU(cudaStreamSynchronize(g->stream));
     FL_CU(cudaMemsetAsync(g->d_flags, 0, sizeof(int), g->stream));
-    if (g->h_status[0] != 0) return FL_OK;
+    FL_CU(cudaStreamSynchronize(g->stream));
+    g->resident = g->h_status[0] == 0;
+    return FL_OK;
+}
+
+// Cuts the terrains into block parts and uploads the plan; again when slope limits, which
+// take room in the blocks, come or go.
+int plan_resident(fl_graph* g) {
+    if (g->d_resident && g->res_slope == g->slope) return FL_OK;
+    const uint32_t blocks = fl::resident_blocks();
+    const uint64_t cap = fl::resident_cap(g->slope);
     // sites per part
-    const uint64_t per = std::min<uint64_t>(cap, std::max<uint64_t>(kResidentPart, (g->n + sms - 1) / sms));
+    const uint64_t per = std::min<uint64_t>(cap, std::max<uint64_t>(kResidentPart, (g->n + blocks - 1) / blocks));
     std::vector<ResidentTerrain> terr(g->terrains);
     std::vector<uint32_t> by_size(g->terrains), slots;
+    g->res_cap = 0;
     for (uint32_t t = 0; t < g->terrains; ++t) {
         const uint32_t m = g->site_off[t + 1] - g->site_off[t];
-        terr[t] = ResidentTerrain{g->site_off[t], m, std::min(sms, (uint32_t)((m + per - 1) / per)), 0};
+        terr[t] = ResidentTerrain{g->site_off[t], m, std::min(blocks, (uint32_t)((m + per - 1) / per)), 0};
         by_size[t] = t;
         g->res_cap = std::max(g->res_cap, (m + terr[t].parts - 1) / terr[t].parts);
     }
@@ -1443,42 +1453,53 @@ int plan_resident(fl_graph* g) {
         slots.insert(slots.end(), terr[t].parts, t);
     }
     g->res_slots = (uint32_t)slots.size();
-    g->res_blocks = std::min(sms, g->res_slots);
+    g->res_blocks = std::min(blocks, g->res_slots);
     const ResidentLayout lay(g->terrains, g->res_slots);
-    FL_TRY(dalloc(&g->d_resident, lay.bytes));
+    if (g->d_resident) {
+        FL_CU(cudaFreeAsync(g->d_resident, g->stream));
+        g->d_resident = nullptr;
+    }
+    FL_CU(cudaMallocAsync((void**)&g->d_resident, lay.bytes, g->stream));
     FL_CU(cudaMemcpyAsync(g->d_resident + lay.terrains, terr.data(), terr.size() * sizeof terr[0],
                           cudaMemcpyHostToDevice, g->stream));
     FL_CU(cudaMemcpyAsync(g->d_resident + lay.slots, slots.data(), slots.size() * 4ull,
                           cudaMemcpyHostToDevice, g->stream));
     FL_CU(cudaStreamSynchronize(g->stream));
-    g->resident = true;
+    g->res_slope = g->slope;
     return FL_OK;
 }
 
 // The largest terrain that the resident solve takes by default.  Its walks go site by site
-// (about 0.6 us a site of the longest river and direction), the staged pass folds whole
+// (about 0.3 us a site of the longest river and direction), the staged pass folds whole
 // chains but pays some 400 us of launches, barriers and skeleton building an iteration.
-// Measured without slope limits (32 iterations, staged / resident, ms): 1,000 sites 4.7 /
-// 0.8, 16,000 12.2 / 5.1, 100,000 16.5 / 12.3, 150,000 17.9 / 17.6, 200,000 19.8 / 21.2.
-// With slope limits the staged walk is site by site too: 65,000 26.4 / 16.0, 400,000 53.5 /
-// 39.5, 600,000 102 / 88.
-constexpr uint32_t kResidentLargest = 131072, kResidentLargestSlope = 524288;
+// Measured without slope limits (32 iterations, staged / resident, ms): 10,000 sites 10.6 /
+// 2.3, 100,000 16.8 / 7.0, 200,000 19.0 / 13.6, 262,000 19.9 / 15.3, 400,000 22.5 / 16.4,
+// 450,000 25.5 / 36.3, 600,000 25.7 / 35.3.  With slope limits the staged walk is site by
+// site too: 100,000 29.5 / 10.5, 600,000 102 / 53.
+constexpr uint32_t kResidentLargest = 262144, kResidentLargestSlope = 786432;
 
 // Whether generate() takes the resident solve: a tuning override of the staged pass's
 // shapes asks for that pass.
 bool use_resident(const fl_graph* g) {
     const fl::Tuning& t = fl::tuning();
-    return g->resident && t.resident != 0 && t.low_ilp < 0 && t.walk_per_sm < 0 &&
+    return g->resident && g->largest <= (uint64_t)fl::resident_blocks() * fl::resident_cap(g->slope) &&
+           t.resident != 0 && t.low_ilp < 0 && t.walk_per_sm < 0 &&
            t.kahn_min_width < 0 && t.sized_grids < 0 &&
            (t.resident == 1 || g->largest <= (g->slope ? kResidentLargestSlope : kResidentLargest));
 }
 
-// The iterations of every terrain from the initial elevations in d_elev; *fell_back when
-// a block met more far donors than it has room for (the model then keeps to the staged
-// pass; d_elev is to be set up again).  iters[t]: iterations of terrain t.
+enum ResidentEnd {
+    kResidentDone,       // every terrain settled or at the limit
+    kResidentNoRoom,     // a block met more far donors than it has room for: the model keeps
+                         // to the staged pass, and d_elev is to be set up again
+    kResidentSlow        // long rivers: the staged pass is to go on from d_elev (one terrain)
+};
+// The iterations of every terrain from the initial elevations in d_elev; iters[t]:
+// iterations of terrain t.
 int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t limit,
-                   std::vector<uint32_t>& iters, bool* fell_back) {
+                   std::vector<uint32_t>& iters, ResidentEnd* end) {
     const uint32_t k = g->terrains;
+    FL_TRY(plan_resident(g));
     const ResidentLayout lay(k, g->res_slots);
     unsigned char* d = g->d_resident;
     FL_CU(cudaMemsetAsync(d + lay.ctrl, 0, sizeof(ResidentCtrl) * k, g->stream));
@@ -1498,6 +1519,8 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     // a launch ends after some tens of milliseconds, so that other streams' solves run
     a.chunk = (uint32_t)std::max<uint64_t>(16, std::min<uint64_t>(1024, (1ull << 27) / std::max(1u, g->n)));
     a.limit = (uint32_t)limit;
+    // about what an iteration of the staged pass takes
+    a.slow_ns = k > 1 || fl::tuning().resident == 1 ? 0 : (400000ull + g->n) * (g->slope ? 2 : 1);
     a.row = g->d_row;
     a.col = g->d_col;
     a.len = g->d_len;
@@ -1518,11 +1541,11 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     a.wl = g->d_wl;
     a.lab = g->d_lab;
     a.lab2 = g->d_lab2;
-    a.root = g->d_sid;
-    a.ef = g->d_t;
     a.best = g->d_best;
-    a.xch = reinterpret_cast<double*>(g->d_trec);
-    a.xch2 = reinterpret_cast<double*>(g->d_rec);
+    a.xtime = reinterpret_cast<double*>(g->d_trec);
+    a.xarea = reinterpret_cast<double*>(g->d_rec);
+    a.xelev = a.xarea + 2ull * g->n;
+    a.troot = g->d_el;
     a.terrains = reinterpret_cast<const ResidentTerrain*>(d + lay.terrains);
     a.slot_terrain = reinterpret_cast<const uint32_t*>(d + lay.slots);
     a.ctrl = reinterpret_cast<ResidentCtrl*>(d + lay.ctrl);
@@ -1548,13 +1571,14 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
         bool need_rank = false;
         for (uint32_t t = 0; t < k; ++t) {
             if (ctrl[t].error == kErrCapacity) {
-                *fell_back = true;
+                *end = kResidentNoRoom;
                 g->resident = false;
                 return FL_OK;
             }
             h[kError] = ctrl[t].error;
             FL_TRY(device_error(h));
-            more |= !ctrl[t].done;
+            if (ctrl[t].slow) *end = kResidentSlow;
+            more |= !ctrl[t].done && !ctrl[t].slow;
             need_rank |= ctrl[t].need_rank != 0;
             iters[t] = ctrl[t].iters;
         }
@@ -1605,26 +1629,28 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
     if (max_iter > 0xffffffffll) max_iter = 0xffffffffll;
     uint64_t limit = max_iter < 0 ? 0xffffffffull : (uint64_t)max_iter;
     uint32_t iters = 0;
+    uint64_t done = 0;                                // iterations of the resident solve
+    FL_CU(cudaEventRecord(g->ev0, g->stream));
     if (limit > 0 && use_resident(g)) {
-        FL_CU(cudaEventRecord(g->ev0, g->stream));
         std::vector<uint32_t> each(g->terrains);
-        bool fell_back = false;
-        FL_TRY(resident_solve(g, outlets, limit, each, &fell_back));
-        if (!fell_back) {
+        ResidentEnd end = kResidentDone;
+        FL_TRY(resident_solve(g, outlets, limit, each, &end));
+        if (end == kResidentDone) {
             for (uint32_t t = 0; t < g->terrains; ++t) {
                 iters = std::max(iters, each[t]);
                 if (terrain_iters) terrain_iters[t] = each[t];
             }
             return finish_generate(g, out_elev, iters, out_iters, loop_ms, total_ms, t_start);
         }
-        FL_TRY(initial_elevations());
+        if (end == kResidentNoRoom) FL_TRY(initial_elevations());
+        else done = each[0];
     }
     // previous-iteration drainage areas steer the skeleton's chain choice; start from
     // the cell areas
     FL_LAUNCH(g, kcMisc, 16.0 * n,
               k_fill_f64<<<blocks_for(n), kThreads, 0, g->stream>>>(n, g->d_A, g->d_area));
     FL_CU(cudaGetLastError());
-    FL_CU(cudaEventRecord(g->ev0, g->stream));
+    if (done == 0) FL_CU(cudaEventRecord(g->ev0, g->stream));   // the loop's time starts here
     g->passes = 0;
     // a terrain alone stops at its first iteration without a change; packed with others
     // it keeps iterating at a fixed point, so its count is that first unchanged iteration
@@ -1649,7 +1675,7 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
         cudaStreamSynchronize(g->stream);
         return rc;
     };
-    uint64_t it = 0;
+    uint64_t it = done;
     bool settled = false;
     for (; it < limit && !settled; ++it) {
         FL_TRY(clear_flags(g));
@@ -1673,7 +1699,7 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
             FL_CU(cudaGetLastError());
         }
         FL_TRY(enqueue_status(g, (int)(it & 1)));
-        if (it > 0) {
+        if (it > done) {
             if (int rc = take_status(g, (int)((it - 1) & 1), h)) return drained(rc);
             if (!h[kChanged]) {                       // iteration it - 1 was the last
                 iters = (uint32_t)it;
@@ -1681,7 +1707,7 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
             }
         }
     }
-    if (!settled && it > 0) {                         // the last iteration's status
+    if (!settled && it > done) {                      // the last iteration's status
         if (int rc = take_status(g, (int)((it - 1) & 1), h)) return drained(rc);
         iters = (uint32_t)it;
     }
@@ -1838,7 +1864,7 @@ int create_graph(uint32_t n, const uint32_t* row_ptr, const uint32_t* col, const
     }
     g->def_outlets.resize(n_default);
     for (uint32_t i = 0; i < n_default; ++i) g->def_outlets[i] = g->inv[default_outlets[i]];
-    if ((rc = plan_resident(g))) return fail(rc);
+    if ((rc = check_resident(g))) return fail(rc);
     *out = g;
     return FL_OK;
 }

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 def _solve(model, params, iters, resident=True):
-    old = _lib.set_tuning(resident=1 if resident else 0)
+    """(elevations, iterations, whether the resident kernel ran); resident None: by the rule."""
+    old = _lib.set_tuning(resident=-1 if resident is None else 1 if resident else 0)
     try:
         g = TerrainGenerator.default().set_model(model).set_parameters(params)
         if iters:
@@ -42,7 +43,7 @@ def _case(n, seed, slope):
 
 
 @pytest.mark.parametrize("slope", [False, True])
-@pytest.mark.parametrize("n", [3, 33, 1023, 1024, 1025, 2049, 5000, 20011, 160001])
+@pytest.mark.parametrize("n", [3, 33, 448, 449, 897, 1025, 2049, 5000, 20011, 160001])
 def test_equals_staged_iterations(n, slope):
     m, p = _case(n, n % 7 + 1, slope)
     iters = 40 if n < 100000 else 6
@@ -92,6 +93,19 @@ def test_caller_order_without_coordinates():
     e, it, _ = _solve(q, r, 5)
     f, jt, staged = _solve(q, r, 5, resident=False)
     assert not staged and it == jt and _same(e, f)
+
+
+def test_long_river_goes_on_in_the_staged_iterations():
+    """A single file of sites is one river as long as the terrain: the resident solve gives up
+    after some iterations and the staged ones go on from there."""
+    n = 20000
+    g = graphs.from_edges(n, [(i, i + 1, 1.0 + 0.25 * (i % 7)) for i in range(n - 1)], default_outlets=[0])
+    m = TerrainModel2D(np.arange(n, dtype=np.float64), np.zeros(n), g.area, g.row_ptr, g.col, g.length,
+                       g.default_outlets)
+    p = ParameterArrays(n, erodibility=np.random.default_rng(1).uniform(0.5, 2.0, n))
+    e, it, used = _solve(m, p, 12, resident=None)
+    f, jt, _ = _solve(m, p, 12, resident=False)
+    assert used and it == jt and _same(e, f)
 
 
 def test_graphs_that_are_not_simple_keep_the_staged_iterations():
