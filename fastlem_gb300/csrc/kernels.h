@@ -232,7 +232,7 @@ void set_last_error(const char* msg);
 // they are (tid / titer null: every site is scanned).
 void launch_receivers(cudaStream_t st, uint32_t n, const uint32_t* row, const uint32_t* col,
                       const double* len, const float* ilen, const double* elev,
-                      const uint8_t* outlet, uint32_t* next, double* rlen, int* flags,
+                      const float2* pair, const uint8_t* outlet, uint32_t* next, double* rlen, int* flags,
                       const uint32_t* tid = nullptr, const uint32_t* titer = nullptr);
 // ilen[s] = 1/len[s] in f32 (NaN where not a normal f32), for launch_receivers.
 void launch_inv_len(cudaStream_t st, uint64_t nnz, const double* len, float* ilen);

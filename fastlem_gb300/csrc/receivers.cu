@@ -5,20 +5,16 @@
 // keeps the first j whose slope is strictly larger than the best so far (starting
 // from 0.0).  The result must be bit-exact, but GB300 issues f64 at 1/64 of the f32
 // rate and a correctly rounded f64 divide costs ~9 f64 operations, which made the
-// straightforward scan FP64-bound.  Here every candidate's slope is first estimated
-// in f32 from the exact bit patterns:
-//   * e_i > e_j is an integer comparison of the bit patterns (both non-negative);
-//   * d = e_i - e_j: when both share a binary exponent (the usual case for
-//     neighbours) the bit patterns' difference is the exact difference in units of
-//     that exponent's ulp, converted to f32 within 2^-23 relative; otherwise it is formed
-//     in 64-bit integers, exactly when the exponents differ by <= 11 and truncated
-//     (error < 2^-52 relative) otherwise, then cut to 24 bits;
-//   * the estimate is d times the slot's 1/len, rounded to f32 once per graph, so it
-//     has relative error below 2^-20.
-// If the largest estimate exceeds every other by more than a factor (1 - 2^-17)^-1,
-// its exact slope is strictly the largest, so it is the reference's receiver.
-// Otherwise (near-ties, negative or non-finite values, values outside the f32
-// range) the row is rescanned exactly as the reference does.
+// straightforward scan FP64-bound.  Here every candidate's slope is first estimated in f32
+// from the elevations' float pairs (slope.cuh), made in a pass before: three additions and a product with the slot's 1/len, within 2^-20 of the
+// slope.  If the largest estimate exceeds every other by more than a factor
+// (1 - 2^-17)^-1, its exact slope is strictly the largest, so it is the reference's
+// receiver.  Otherwise (near-ties, differences below 2^-24 of the elevation, non-finite or
+// out-of-range values) the row is rescanned exactly as the reference does.
+// The scan is bound by instruction issue and the gathers' latency.  Estimates from the two
+// doubles' bit patterns (64-bit subtraction, exponent checks and two conversions a slot)
+// took 710 us at 16M sites and 57 us at 1M; the scan now takes 515 us and 43 us, the pairs'
+// own pass 51 us and 7 us.
 
 #include <algorithm>
 #include <cfloat>
@@ -40,64 +36,38 @@ __device__ __forceinline__ void scan_site(uint32_t i, uint32_t s0, uint32_t s1, 
                                           const double* __restrict__ len,
                                           const float* __restrict__ ilen,
                                           const double* __restrict__ elev,
+                                          const float2* __restrict__ pair,
                                           uint32_t* __restrict__ next, double* __restrict__ rlen,
                                           bool* lake, bool* went_exact) {
-    const double ei = elev[i];
-    const uint64_t EI = (uint64_t)__double_as_longlong(ei);
-    bool exact = (EI >> 63) != 0 || (EI >> 52) == 0x7ff;   // negative or non-finite
-    float best = 0.0f, second = 0.0f;
-    uint32_t best_slot = kNone;
-    bool any_lower = false;
-    if (!exact) {
-        // one candidate: exact comparison of the bit patterns, then the f32 estimate
-        auto consider = [&](uint32_t s, uint64_t EJ) {
-            if (exact) return;
-            if ((EJ >> 63) || (EJ >> 52) == 0x7ff) { exact = true; return; }
-            if (EI <= EJ) return;                          // not lower (bits are monotone)
-            any_lower = true;
-            float d;
-            if (!slope_diff(EI, EJ, d)) {
-                exact = true;
-                return;
-            }
-            const float a = d * ilen[s];
-            if (!(a > 1e-30f) || !(a < 1e30f)) { exact = true; return; }
-            if (a > best) {
-                second = best;
-                best = a;
-                best_slot = s;
-            } else if (a > second) {
-                second = a;
-            }
-        };
-        const uint32_t deg = s1 - s0;
-        if (deg <= (uint32_t)kRowFast) {
-            // short rows: all neighbour elevations in flight at once
-            uint32_t jj[kRowFast];
-            uint64_t ej[kRowFast];
+    PairScan sc(pair[i]);
+    const uint32_t deg = s1 - s0;
+    if (deg <= (uint32_t)kRowFast) {
+        // short rows: all neighbour elevations in flight at once
+        uint32_t jj[kRowFast];
+        float2 ej[kRowFast];
 #pragma unroll
-            for (int k = 0; k < kRowFast; ++k) {
-                if ((uint32_t)k >= dmax) break;
-                if ((uint32_t)k < deg) jj[k] = col[s0 + k];
-            }
-#pragma unroll
-            for (int k = 0; k < kRowFast; ++k) {
-                if ((uint32_t)k >= dmax) break;
-                if ((uint32_t)k < deg) ej[k] = (uint64_t)__double_as_longlong(elev[jj[k]]);
-            }
-#pragma unroll
-            for (int k = 0; k < kRowFast; ++k) {
-                if ((uint32_t)k >= dmax) break;
-                if ((uint32_t)k < deg) consider(s0 + k, ej[k]);
-            }
-        } else {
-            for (uint32_t s = s0; s < s1; ++s)
-                consider(s, (uint64_t)__double_as_longlong(elev[col[s]]));
+        for (int k = 0; k < kRowFast; ++k) {
+            if ((uint32_t)k >= dmax) break;
+            if ((uint32_t)k < deg) jj[k] = col[s0 + k];
         }
-        if (!exact && any_lower && second > best * (1.0f - 7.62939453125e-06f)) exact = true;
+#pragma unroll
+        for (int k = 0; k < kRowFast; ++k) {
+            if ((uint32_t)k >= dmax) break;
+            if ((uint32_t)k < deg) ej[k] = pair[jj[k]];
+        }
+#pragma unroll
+        for (int k = 0; k < kRowFast; ++k) {
+            if ((uint32_t)k >= dmax) break;
+            if ((uint32_t)k < deg) sc.consider(s0 + k, ej[k], ilen[s0 + k]);
+        }
+    } else {
+        for (uint32_t s = s0; s < s1; ++s) sc.consider(s, pair[col[s]], ilen[s]);
     }
+    uint32_t best_slot = sc.slot;
+    const bool exact = !sc.decided();
     if (exact) {
         *went_exact = true;
+        const double ei = elev[i];
         double steepest = 0.0;
         best_slot = kNone;
         for (uint32_t s = s0; s < s1; ++s) {
@@ -129,7 +99,7 @@ __device__ __forceinline__ void scan_site(uint32_t i, uint32_t s0, uint32_t s1, 
 __global__ void k_receivers(uint32_t n, const uint32_t* __restrict__ row,
                             const uint32_t* __restrict__ col, const double* __restrict__ len,
                             const float* __restrict__ ilen, const double* __restrict__ elev,
-                            const uint8_t* __restrict__ outlet, uint32_t* __restrict__ next,
+                            const float2* __restrict__ pair, const uint8_t* __restrict__ outlet, uint32_t* __restrict__ next,
                             double* __restrict__ rlen, int* __restrict__ flags,
                             const uint32_t* __restrict__ tid, const uint32_t* __restrict__ titer) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -148,7 +118,7 @@ __global__ void k_receivers(uint32_t n, const uint32_t* __restrict__ row,
     }
     const uint32_t deg = s1 - s0;
     const uint32_t dmax = __reduce_max_sync(0xffffffffu, deg <= (uint32_t)kRowFast ? deg : 0u);
-    if (scan) scan_site(i, s0, s1, dmax, col, len, ilen, elev, next, rlen, &lake, &went_exact);
+    if (scan) scan_site(i, s0, s1, dmax, col, len, ilen, elev, pair, next, rlen, &lake, &went_exact);
     block_flag(flags, kHasLake, lake);
     if (__syncthreads_or(went_exact) && threadIdx.x == 0) atomicAdd(&flags[kExact], 1);
 }
@@ -167,10 +137,10 @@ __global__ void k_inv_len(uint64_t nnz, const double* __restrict__ len, float* _
 
 void launch_receivers(cudaStream_t st, uint32_t n, const uint32_t* row, const uint32_t* col,
                       const double* len, const float* ilen, const double* elev,
-                      const uint8_t* outlet, uint32_t* next, double* rlen, int* flags,
+                      const float2* pair, const uint8_t* outlet, uint32_t* next, double* rlen, int* flags,
                       const uint32_t* tid, const uint32_t* titer) {
     k_receivers<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(
-        n, row, col, len, ilen, elev, outlet, next, rlen, flags, tid && titer ? tid : nullptr, titer);
+        n, row, col, len, ilen, elev, pair, outlet, next, rlen, flags, tid && titer ? tid : nullptr, titer);
 }
 
 void launch_inv_len(cudaStream_t st, uint64_t nnz, const double* len, float* ilen) {

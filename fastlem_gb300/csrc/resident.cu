@@ -157,10 +157,10 @@ __device__ __noinline__ uint32_t steepest_exact(const uint32_t* row, const uint3
     double top = 0.0;
     uint32_t slot = kNone;
 #pragma unroll 1
-    for (uint32_t s = row[g], e = row[g + 1]; s < e; ++s) {
-        const double ej = elev[col[s]];
+    for (uint32_t s = __ldg(&row[g]), e = __ldg(&row[g + 1]); s < e; ++s) {
+        const double ej = elev[__ldg(&col[s])];
         if (ei > ej) {
-            const double m = __ddiv_rn(__dsub_rn(ei, ej), len[s]);
+            const double m = __ddiv_rn(__dsub_rn(ei, ej), __ldg(&len[s]));
             if (m > top) {
                 top = m;
                 slot = s;
@@ -173,7 +173,7 @@ __device__ __noinline__ uint32_t steepest_exact(const uint32_t* row, const uint3
 // The steepest-descent receiver of site g from the elevations' float pairs (slope.cuh):
 // its slot, or kNone.
 __device__ __forceinline__ uint32_t steepest(const ResidentArgs& a, uint32_t g) {
-    const uint32_t s0 = a.row[g], s1 = a.row[g + 1];
+    const uint32_t s0 = __ldg(&a.row[g]), s1 = __ldg(&a.row[g + 1]);
     const float2 own = a.pair[g];
     PairScan sc(own);
 #pragma unroll 1
@@ -183,8 +183,8 @@ __device__ __forceinline__ uint32_t steepest(const ResidentArgs& a, uint32_t g) 
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const uint32_t s = min(b + k, s1 - 1);
-            e[k] = a.pair[a.col[s]];
-            f[k] = a.ilen[s];
+            e[k] = a.pair[__ldg(&a.col[s])];
+            f[k] = __ldg(&a.ilen[s]);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -194,8 +194,16 @@ __device__ __forceinline__ uint32_t steepest(const ResidentArgs& a, uint32_t g) 
 }
 
 __device__ __forceinline__ double edge_or_one(const ResidentArgs& a, uint32_t i, uint32_t j) {
-    for (uint32_t s = a.row[i], e = a.row[i + 1]; s < e; ++s)
-        if (a.col[s] == j) return a.len[s];
+    const uint32_t s0 = __ldg(&a.row[i]), e = __ldg(&a.row[i + 1]);
+#pragma unroll 1
+    for (uint32_t s = s0; s < e; s += 4) {               // four columns in flight
+        uint32_t c[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[k] = __ldg(&a.col[min(s + k, e - 1)]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (s + k < e && c[k] == j) return __ldg(&a.len[s + k]);
+    }
     return 1.0;
 }
 
@@ -231,13 +239,13 @@ __device__ __noinline__ void reroute_lakes(const ResidentArgs& a, Group& gr, uin
     if (!gr.ok) return;
 #pragma unroll 1
     for (uint32_t v = threadIdx.x; v < S; v += blockDim.x) {
-        const uint32_t g = lo + v, r = a.rank[g];
+        const uint32_t g = lo + v, r = __ldg(&a.rank[g]);
         if (r == kNone) continue;
         const uint32_t own = __ldcg(&cur[g]);
-        const uint32_t s0 = a.row[g], s1 = a.row[g + 1];
+        const uint32_t s0 = __ldg(&a.row[g]), s1 = __ldg(&a.row[g + 1]);
         for (uint32_t s = s0; s < s1; ++s) {
-            const uint32_t L = __ldcg(&cur[a.col[s]]);
-            if (a.outlet[L] || L == own) continue;
+            const uint32_t L = __ldcg(&cur[__ldg(&a.col[s])]);
+            if (__ldg(&a.outlet[L]) || L == own) continue;
             const unsigned long long key = ((unsigned long long)r << 32) | (s - s0);
             if (key < __ldcg(&a.best[L])) atomicMin(&a.best[L], key);
         }
@@ -249,8 +257,8 @@ __device__ __noinline__ void reroute_lakes(const ResidentArgs& a, Group& gr, uin
     for (uint32_t v = threadIdx.x; v < S; v += blockDim.x) {
         const unsigned long long key = __ldcg(&a.best[lo + v]);
         if (key == kNoKey) continue;
-        uint32_t nk = a.sor[key >> 32];
-        uint32_t k = a.col[a.row[nk] + (uint32_t)key];
+        uint32_t nk = __ldg(&a.sor[key >> 32]);
+        uint32_t k = __ldg(&a.col[__ldg(&a.row[nk]) + (uint32_t)key]);
         for (uint32_t steps = 0;; ++steps) {
             if (steps > a.n) {
                 raise(gr.ctrl, kErrForest);
@@ -427,10 +435,10 @@ template <bool kSlope>
 __device__ __noinline__ double add_long(const ResidentArgs& a, uint32_t lo, uint32_t S, uint32_t nfar,
                                         uint32_t v, double x) {
     const Block bk = carve<kSlope>(a.cap);
-    const uint32_t g = lo + v, s0 = a.row[g];
+    const uint32_t g = lo + v, s0 = __ldg(&a.row[g]);
 #pragma unroll 1
-    for (uint32_t s = a.row[g + 1]; s-- > s0;) {
-        const uint32_t j = a.col[s], d = j - lo;
+    for (uint32_t s = __ldg(&a.row[g + 1]); s-- > s0;) {
+        const uint32_t j = __ldg(&a.col[s]), d = j - lo;
         if (d < S) {
             const uint32_t w = lds32(bk.word(d));
             if (!(w & (kRoot | kFar)) && (w >> kParentShift) == v) x = __dadd_rn(x, ldsd(bk.rec(d)));
@@ -578,15 +586,15 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
                 if (kSlope) st_relaxed64(elev_slot(a, g, par ^ 1u), kPendingBits);
             }
             uint32_t slot = kNone;
-            if (!a.outlet[g]) {
+            if (!__ldg(&a.outlet[g])) {
                 slot = steepest(a, g);
                 lake |= slot == kNone;
             }
-            const uint32_t p = slot == kNone ? g : a.col[slot];
+            const uint32_t p = slot == kNone ? g : __ldg(&a.col[slot]);
             a.next[g] = p;
-            a.rlen[g] = slot == kNone ? 1.0 : a.len[slot];
+            a.rlen[g] = slot == kNone ? 1.0 : __ldg(&a.len[slot]);
             note(v, p);
-            stsd(bk.rec(v), a.area[g]);
+            stsd(bk.rec(v), __ldg(&a.area[g]));
         }
         const bool lakes = group_barrier(gr, lake);
         if (!gr.ok) break;
@@ -608,7 +616,7 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
             bool leaf = false, out = false;
             if (v < S) {
                 const uint32_t g = lo + v;
-                const uint32_t s0 = a.row[g], s1 = a.row[g + 1];
+                const uint32_t s0 = __ldg(&a.row[g]), s1 = __ldg(&a.row[g + 1]);
                 uint32_t cnt = 0, kind = 0;
                 uint64_t dn = (uint64_t)bk.none * 0x0001000100010001ull;
 #pragma unroll 1
@@ -616,7 +624,7 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
                     uint32_t j[4];
                     bool don[4];
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) j[k] = a.col[max(hi, s0 + 1 + k) - 1 - k];
+                    for (int k = 0; k < 4; ++k) j[k] = __ldg(&a.col[max(hi, s0 + 1 + k) - 1 - k]);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {
                         const uint32_t d = j[k] - lo;
@@ -763,7 +771,7 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
         for (uint32_t i = tid; i < nlist; i += kT) {
             const uint32_t u = lds16(bk.list + 2 * i), g = lo + u;
             const double A = ldsd(bk.rec(u)), l = __ldcg(&a.rlen[g]);
-            const double cel = __dmul_rn(a.k[g], __dsqrt_rn(A));
+            const double cel = __dmul_rn(__ldg(&a.k[g]), __dsqrt_rn(A));
             a.w[g] = __dmul_rn(__ddiv_rn(1.0, cel), l);
             a.wa[g] = A;
             a.wl[g] = l;
@@ -781,12 +789,12 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
                 continue;
             }
             const double t = plus_zero(plus_zero(wv));
-            const bool out = a.outlet[g] != 0;
+            const bool out = __ldg(&a.outlet[g]) != 0;
             if (out) {
                 const double old_e = __ldcg(&a.elev[g]), dt = __dsub_rn(t, t);
-                double ne = __dadd_rn(old_e, __dmul_rn(a.u[g], dt > 0.0 ? dt : 0.0));
+                double ne = __dadd_rn(old_e, __dmul_rn(__ldg(&a.u[g]), dt > 0.0 ? dt : 0.0));
                 if (kSlope) {
-                    const double tn = a.tanms[g], dist = __ldcg(&a.rlen[g]);
+                    const double tn = __ldg(&a.tanms[g]), dist = __ldcg(&a.rlen[g]);
                     if (!isnan(tn) && __ddiv_rn(__dsub_rn(ne, old_e), dist) > tn)
                         ne = __dadd_rn(old_e, __dmul_rn(tn, dist));
                 }
@@ -814,7 +822,7 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
             if (!(r & kNoOutlet) && !is_root) {
                 const double to = __ldcg(root_time(a, r)), eo = __ldcg(&a.elev[r]);
                 const double dt = __dsub_rn(ldsd(rec), to);
-                ne = __dadd_rn(eo, __dmul_rn(a.u[g], dt > 0.0 ? dt : 0.0));
+                ne = __dadd_rn(eo, __dmul_rn(__ldg(&a.u[g]), dt > 0.0 ? dt : 0.0));
                 if (!kSlope) {
                     changed |= ne != __ldcg(&a.elev[g]);
                     a.elev[g] = ne;
@@ -826,7 +834,7 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
             if (kSlope) {
                 // tan * len, or a negative number where there is no limit or the product
                 // cannot stand in for the quotient
-                const double tn = a.tanms[g], dist = __ldcg(&a.rlen[g]), rise = __dmul_rn(tn, dist);
+                const double tn = __ldg(&a.tanms[g]), dist = __ldcg(&a.rlen[g]), rise = __dmul_rn(tn, dist);
                 stsd(bk.lim + 8 * u, tn > 1e-200 && dist > 0.0 && rise > 1e-200 && rise < 1e200 && !(r & kNoOutlet) ? rise : -1.0);
                 if (is_root && (lds32(bk.word(u)) & kFarDonor)) st_relaxed64(elev_slot(a, g, par), published(ne));
                 sts128(rec, bits(ne), (uint64_t)(is_root ? 2 : 1) << 32 | r);

@@ -54,53 +54,4 @@ struct PairScan {
     }
 };
 
-// ---- estimates from the bit patterns of two doubles (the bounds are in receivers.cu) --
-constexpr uint64_t kMant = (1ull << 52) - 1;
-// Float estimate of (a - b) for non-negative finite doubles with bits A > B.
-// Returns false when the result falls outside the normal f32 range.
-__device__ __forceinline__ bool diff_estimate(uint64_t A, uint64_t B, float& out) {
-    int ea = (int)(A >> 52), eb = (int)(B >> 52);
-    uint64_t ma = (A & kMant) | (ea ? (1ull << 52) : 0);
-    uint64_t mb = (B & kMant) | (eb ? (1ull << 52) : 0);
-    ea = ea ? ea : 1;
-    eb = eb ? eb : 1;
-    int sh = ea - eb;
-    uint64_t D;
-    int E;
-    if (sh <= 11) {
-        D = (ma << sh) - mb;
-        E = eb;
-    } else {
-        D = ma - (sh < 64 ? (mb >> sh) : 0);
-        E = ea;
-    }
-    if (D == 0) return false;
-    int lz = __clzll((long long)D);
-    uint64_t top = D << lz;                      // leading one at bit 63
-    int e2 = (63 - lz) + E - 1075;               // d = 1.xxx * 2^e2
-    int fe = e2 + 127;
-    if (fe <= 0 || fe >= 255) return false;
-    uint32_t fb = ((uint32_t)fe << 23) | (uint32_t)((top >> 40) & 0x7fffffu);
-    out = __uint_as_float(fb);
-    return true;
-}
-
-// f32 estimate of a - b for non-negative finite doubles with bits A > B.  Sharing
-// the exponent field e in [949, 1149], A - B is the difference in units of 2^(e-1075)
-// (below 2^52) and the scaled result is a normal f32 number.  The 52-bit difference is
-// converted as two 32-bit halves (a 64-bit integer conversion issues on the f64 pipe):
-// the high half is exact, the low half truncated and the fused sum rounded, within
-// 2^-23 relative.
-__device__ __forceinline__ bool slope_diff(uint64_t A, uint64_t B, float& out) {
-    const uint32_t e = (uint32_t)(A >> 52);
-    if (e == (uint32_t)(B >> 52) && e - 949u <= 200u) {
-        const uint64_t D = A - B;
-        const float d = fmaf(__uint2float_rz((uint32_t)(D >> 32)), 4294967296.0f,
-                             __uint2float_rz((uint32_t)D));
-        out = d * __uint_as_float((e - 948u) << 23);
-        return true;
-    }
-    return diff_estimate(A, B, out);
-}
-
 }  // namespace fl

@@ -143,6 +143,14 @@ __global__ void k_initial_elevation(uint32_t n, const uint32_t* __restrict__ per
     pair[j] = float_pair(e);
 }
 
+// The elevations' float pairs.  A pass of its own over the elevations in memory order (16 B a
+// site): written beside the elevations by the top-down rounds, whose order scatters them,
+// they cost 240 us an iteration at 16M sites.
+__global__ void k_pairs(uint32_t n, const double* __restrict__ elev, float2* __restrict__ pair) {
+    uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j < n) pair[j] = float_pair(elev[j]);
+}
+
 // dst[j] = src[idx[j]]: caller order <-> device order.
 __global__ void k_gather_f64(uint32_t n, const uint32_t* __restrict__ idx,
                              const double* __restrict__ src, double* __restrict__ dst) {
@@ -168,8 +176,15 @@ __device__ __forceinline__ double edge_len_or_one(const uint32_t* __restrict__ r
                                                   const uint32_t* __restrict__ col,
                                                   const double* __restrict__ len, uint32_t i,
                                                   uint32_t j) {
-    for (uint32_t s = row[i], e = row[i + 1]; s < e; ++s)
-        if (col[s] == j) return len[s];
+    const uint32_t s0 = __ldg(&row[i]), e = __ldg(&row[i + 1]);
+    for (uint32_t s = s0; s < e; s += 4) {               // four columns in flight
+        uint32_t c[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) c[k] = __ldg(&col[min(s + k, e - 1)]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (s + k < e && c[k] == j) return __ldg(&len[s + k]);
+    }
     return 1.0;
 }
 
@@ -178,25 +193,86 @@ __global__ void k_copy_u32(uint32_t n, const uint32_t* __restrict__ a, uint32_t*
     if (i < n) b[i] = a[i];
 }
 
-// Basin labels of the receivers by pointer jumping, every round in one cooperative
-// launch: lab = next, then lab[i] = lab[lab[i]] until no label moves.  Roots
-// (next[r] == r) are fixed points, so after ceil(log2(depth)) rounds every site holds
-// its basin root (stream_tree.rs:139-173, "subroot"); the rounds synchronise on the
-// grid barrier and a rotating "moved" word, and the result ends in lab.  With a gate,
-// nothing runs unless *gate is set (the receivers found a lake), so the launch can be
-// enqueued before the host knows.
-__global__ void k_labels(uint32_t n, const uint32_t* __restrict__ next, uint32_t* lab,
-                         uint32_t* lab2, const int* gate, int* flags) {
-    if (gate && *gate == 0) return;                      // the same verdict for every block
+struct LakeArgs {
+    uint32_t n;
+    const uint32_t *row, *col;
+    const double* len;
+    uint32_t* next;
+    double* rlen;
+    uint32_t *lab, *lab2;
+    unsigned long long* best;
+    const uint32_t *rank, *sor;
+    const uint8_t* outlet;
+    const int* gate;
+    int* flags;
+    bool reroute;            // keys and flips follow the labels
+};
+
+// Keys: for site v the lake heap processes (rank[v] != none) and every neighbour j lying in a
+// lake L other than v's own basin, best[L] = min((rank[v] << 32) | slot).  The minimum is the
+// first processed site touching L and, within its row, the first entry in L -- the pair at
+// which the reference flips L (stream_tree.rs:204-230).
+__device__ __forceinline__ void lake_keys(const LakeArgs& a, const uint32_t* lab, uint32_t v) {
+    const uint32_t r = __ldg(&a.rank[v]);
+    if (r == kNone) return;
+    const uint32_t lv = lab[v];
+    const uint32_t s0 = __ldg(&a.row[v]), s1 = __ldg(&a.row[v + 1]);
+    for (uint32_t s = s0; s < s1; ++s) {
+        const uint32_t L = lab[__ldg(&a.col[s])];
+        if (__ldg(&a.outlet[L]) || L == lv) continue;
+        const unsigned long long key = ((unsigned long long)r << 32) | (unsigned long long)(s - s0);
+        if (key < a.best[L]) atomicMin(&a.best[L], key);
+    }
+}
+
+// Flips: reverses lake L's receiver path from j* to the lake bottom and hangs it on v*
+// (stream_tree.rs:214-228).  Lakes are disjoint and each flip only touches its own lake's
+// sites, so lakes run independently.
+__device__ __forceinline__ void lake_flip(const LakeArgs& a, uint32_t L) {
+    const unsigned long long key = __ldcg(&a.best[L]);
+    if (key == kNoKey) return;
+    const uint32_t v = __ldg(&a.sor[key >> 32]);
+    uint32_t k = __ldg(&a.col[__ldg(&a.row[v]) + (uint32_t)(key & 0xffffffffu)]), nk = v;
+    uint32_t nx = a.next[k];
+    for (uint32_t steps = 0;; ++steps) {
+        if (steps > a.n) {           // a cycle: cannot happen on a descent forest
+            set_error(a.flags, kErrForest);
+            return;
+        }
+        const uint32_t after = a.next[nx];               // in flight over the row's scan
+        const double d = edge_len_or_one(a.row, a.col, a.len, k, nk);
+        a.next[k] = nk;
+        a.rlen[k] = d;
+        if (nx == k) return;
+        nk = k;
+        k = nx;
+        nx = after;
+    }
+}
+
+// Basin labels, and with reroute the whole lake re-routing, in one cooperative launch.  With
+// a gate, nothing runs unless *gate is set (the receivers found a lake), so the launch can
+// be enqueued before the host knows.
+// Labels by pointer jumping: lab = next, then lab[i] = lab[lab[i]] until no label moves.
+// Roots (next[r] == r) are fixed points, so after ceil(log2(depth)) rounds every site holds
+// its basin root (stream_tree.rs:139-173, "subroot"); the rounds synchronise on the grid
+// barrier and a rotating "moved" word, and the result ends in lab.
+__global__ void __launch_bounds__(1024, 2) k_lakes(LakeArgs a) {
+    if (a.gate && *a.gate == 0) return;                  // the same verdict for every block
+    const uint32_t n = a.n;
     const uint32_t gtid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = gtid; i < n; i += stride) lab[i] = next[i];
-    if (!grid_barrier(flags)) return;
-    uint32_t* cur = lab;
-    uint32_t* out = lab2;
-    for (uint32_t round = 0; round < 64; ++round) {
-        int* moved_word = &flags[kJump0 + round % 3];
-        if (gtid == 0) flags[kJump0 + (round + 1) % 3] = 0;
+    for (uint32_t i = gtid; i < n; i += stride) {
+        a.lab[i] = a.next[i];
+        a.best[i] = kNoKey;
+    }
+    if (!grid_barrier(a.flags)) return;
+    uint32_t* cur = a.lab;
+    uint32_t* out = a.lab2;
+    bool more = true;
+    for (uint32_t round = 0; more && round < 64; ++round) {
+        int* moved_word = &a.flags[kJump0 + round % 3];
+        if (gtid == 0) a.flags[kJump0 + (round + 1) % 3] = 0;
         bool moved = false;
         for (uint32_t i = gtid; i < n; i += stride) {
             const uint32_t l = __ldcg(&cur[i]);
@@ -205,80 +281,24 @@ __global__ void k_labels(uint32_t n, const uint32_t* __restrict__ next, uint32_t
             moved |= ll != l;
         }
         if (__syncthreads_or(moved) && threadIdx.x == 0) atomicOr(moved_word, 1);
-        if (!grid_barrier(flags)) return;
+        if (!grid_barrier(a.flags)) return;
         uint32_t* t = cur;
         cur = out;
         out = t;
-        if (ld_acquire(moved_word) == 0) {
-            if (cur != lab)
-                for (uint32_t i = gtid; i < n; i += stride) lab[i] = __ldcg(&cur[i]);
-            return;
-        }
+        more = ld_acquire(moved_word) != 0;
     }
-    if (gtid == 0) set_error(flags, kErrForest);          // a receiver cycle
-}
-
-// best[L] = no key, for every site (gated like k_labels).
-__global__ void k_clear_keys(uint32_t n, unsigned long long* __restrict__ best,
-                             const int* gate) {
-    if (gate && *gate == 0) return;
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) best[i] = kNoKey;
-}
-
-// For every site v the lake heap processes (rank[v] != none) and every neighbour j
-// lying in a lake L other than v's own basin: best[L] = min((rank[v] << 32) | slot).
-// The minimum is the first processed site touching L and, within its row, the
-// first entry in L -- the pair at which the reference flips L (stream_tree.rs:204-230).
-__global__ void k_lake_keys(uint32_t n, const uint32_t* __restrict__ row,
-                            const uint32_t* __restrict__ col, const uint32_t* __restrict__ rank,
-                            const uint32_t* __restrict__ lab, const uint8_t* __restrict__ outlet,
-                            unsigned long long* __restrict__ best, const int* gate) {
-    if (gate && *gate == 0) return;
-    uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (v >= n) return;
-    uint32_t r = rank[v];
-    if (r == kNone) return;
-    uint32_t lv = lab[v];
-    const uint32_t s0 = row[v], s1 = row[v + 1];
-    for (uint32_t s = s0; s < s1; ++s) {
-        uint32_t L = lab[col[s]];
-        if (outlet[L] || L == lv) continue;
-        unsigned long long key = ((unsigned long long)r << 32) | (unsigned long long)(s - s0);
-        if (key < best[L]) atomicMin(&best[L], key);
+    if (more) {                                          // a receiver cycle
+        if (gtid == 0) set_error(a.flags, kErrForest);
+        return;
     }
-}
-
-// One thread per lake: reverse the receiver path from j* to the lake bottom and
-// hang it on v* (stream_tree.rs:214-228).  Lakes are disjoint and each flip only
-// touches its own lake's sites, so lakes run independently.
-__global__ void k_lake_flip(uint32_t n, const uint32_t* __restrict__ row,
-                            const uint32_t* __restrict__ col, const double* __restrict__ len,
-                            const unsigned long long* __restrict__ best,
-                            const uint32_t* __restrict__ site_of_rank, uint32_t* next,
-                            double* rlen, int* flags, const int* gate) {
-    if (gate && *gate == 0) return;
-    uint32_t L = blockIdx.x * blockDim.x + threadIdx.x;
-    if (L >= n) return;
-    unsigned long long key = best[L];
-    if (key == kNoKey) return;
-    uint32_t v = site_of_rank[key >> 32];
-    uint32_t j = col[row[v] + (uint32_t)(key & 0xffffffffu)];
-    uint32_t k = j, nk = v;
-    for (uint32_t steps = 0;; ++steps) {
-        if (steps > n) {             // a cycle: cannot happen on a descent forest
-            set_error(flags, kErrForest);
-            return;
-        }
-        uint32_t nx = next[k];
-        if (nx == k) break;
-        next[k] = nk;
-        rlen[k] = edge_len_or_one(row, col, len, k, nk);
-        nk = k;
-        k = nx;
+    if (!a.reroute) {
+        if (cur != a.lab)
+            for (uint32_t i = gtid; i < n; i += stride) a.lab[i] = __ldcg(&cur[i]);
+        return;
     }
-    next[k] = nk;
-    rlen[k] = edge_len_or_one(row, col, len, k, nk);
+    for (uint32_t v = gtid; v < n; v += stride) lake_keys(a, cur, v);
+    if (!grid_barrier(a.flags)) return;
+    for (uint32_t L = gtid; L < n; L += stride) lake_flip(a, L);
 }
 
 __global__ void k_fill_nan(uint32_t n, double* __restrict__ d) {
@@ -1158,44 +1178,32 @@ int set_outlets(fl_graph* g, const std::vector<uint32_t>& outlets, bool need_ran
 
 // Receivers for the current elevations; the kernel raises flags[kHasLake].
 int enqueue_receivers(fl_graph* g) {
+    FL_LAUNCH(g, kcReceivers, 16.0 * g->n,
+              k_pairs<<<blocks_for(g->n), kThreads, 0, g->stream>>>(g->n, g->d_elev, g->d_pair));
     FL_LAUNCH(g, kcReceivers, 25.0 * g->n + 20.0 * g->nnz,
               fl::launch_receivers(g->stream, g->n, g->d_row, g->d_col, g->d_len, g->d_ilen,
-                                   g->d_elev, g->d_outlet, g->d_next, g->d_rlen, g->d_flags,
+                                   g->d_elev, g->d_pair, g->d_outlet, g->d_next, g->d_rlen, g->d_flags,
                                    g->d_tid, g->d_titer));
     FL_CU(cudaGetLastError());
     return FL_OK;
 }
 
-// Basin labels of d_next into d_lab (pointer jumping, one cooperative launch); with a
-// gate, only if *gate is set when the kernel runs.
-int enqueue_labels(fl_graph* g, const int* gate) {
-    uint32_t n = g->n;
-    static const unsigned full = coop_blocks((const void*)k_labels, 1024, 2);
+// Basin labels of d_next into d_lab and, with reroute, lake re-routing on d_next; with a
+// gate, only if *gate is set when the kernel runs.  One launch: each that skips itself, as in
+// most iterations, takes 5 to 7 us (30 us an iteration for four at 1M sites, 9.6 for one),
+// and the lakes of a 16M-site terrain's first iteration take 0.95 ms against 1.85 in four.
+int enqueue_lakes(fl_graph* g, const int* gate, bool reroute) {
+    const uint32_t n = g->n;
+    static const unsigned full = coop_blocks((const void*)k_lakes, 1024, 2);
     const bool sized = g->sized_grids >= 0 ? g->sized_grids != 0
                                            : fl::shape_for(n, g->terrains > 1).sized_grids;
     const unsigned grid = fl::sized_grid(sized, full, n, 1024 * 8);
-    const int* gt = gate;
-    void* argv[] = {(void*)&n, (void*)&g->d_next, (void*)&g->d_lab, (void*)&g->d_lab2,
-                    (void*)&gt, (void*)&g->d_flags};
-    FL_LAUNCH(g, kcLakes, 8.0 * n,
-              cudaLaunchCooperativeKernel((const void*)k_labels, dim3(grid), dim3(1024), argv, 0,
+    LakeArgs a{n, g->d_row, g->d_col, g->d_len, g->d_next, g->d_rlen, g->d_lab, g->d_lab2, g->d_best,
+               g->d_rank, g->d_sor, g->d_outlet, gate, g->d_flags, reroute};
+    void* argv[] = {(void*)&a};
+    FL_LAUNCH(g, kcLakes, 16.0 * n + (reroute ? 20.0 * n + 8.0 * g->nnz : 0.0),
+              cudaLaunchCooperativeKernel((const void*)k_lakes, dim3(grid), dim3(1024), argv, 0,
                                           g->stream));
-    FL_CU(cudaGetLastError());
-    return FL_OK;
-}
-
-// Lake re-routing on d_next (labels must be current), gated like enqueue_labels.
-int enqueue_lakes(fl_graph* g, const int* gate) {
-    uint32_t n = g->n;
-    FL_LAUNCH(g, kcLakes, 8.0 * n,
-              k_clear_keys<<<blocks_for(n), kThreads, 0, g->stream>>>(n, g->d_best, gate));
-    FL_LAUNCH(g, kcLakes, 12.0 * n + 8.0 * g->nnz,
-              k_lake_keys<<<blocks_for(n), kThreads, 0, g->stream>>>(
-                  n, g->d_row, g->d_col, g->d_rank, g->d_lab, g->d_outlet, g->d_best, gate));
-    FL_LAUNCH(g, kcLakes, 8.0 * n,
-              k_lake_flip<<<blocks_for(n), kThreads, 0, g->stream>>>(
-                  n, g->d_row, g->d_col, g->d_len, g->d_best, g->d_sor, g->d_next, g->d_rlen,
-                  g->d_flags, gate));
     FL_CU(cudaGetLastError());
     return FL_OK;
 }
@@ -1688,10 +1696,7 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
             gate = nullptr;
             if (lakes) FL_TRY(set_outlets(g, outlets, true));
         }
-        if (lakes) {
-            FL_TRY(enqueue_labels(g, gate));
-            FL_TRY(enqueue_lakes(g, gate));
-        }
+        if (lakes) FL_TRY(enqueue_lakes(g, gate, true));
         FL_TRY(enqueue_basin_pass(g));
         if (g->d_titer) {
             k_terrain_iters<<<blocks_for(g->terrains), kThreads, 0, g->stream>>>(
@@ -2030,10 +2035,10 @@ int fl_probe_lakes(fl_graph* g, const uint32_t* outlets, uint32_t n_outlets,
     FL_CU(cudaMemcpyAsync(g->d_next, nx.data(), n * 4ull, cudaMemcpyHostToDevice, g->stream));
     std::vector<double> ones(n, 1.0);
     FL_CU(cudaMemcpyAsync(g->d_rlen, ones.data(), n * 8ull, cudaMemcpyHostToDevice, g->stream));
-    FL_TRY(enqueue_labels(g, nullptr));
+    FL_TRY(enqueue_lakes(g, nullptr, false));
     std::vector<uint32_t> lab(n);
     FL_CU(cudaMemcpyAsync(lab.data(), g->d_lab, n * 4ull, cudaMemcpyDeviceToHost, g->stream));
-    FL_TRY(enqueue_lakes(g, nullptr));
+    FL_TRY(enqueue_lakes(g, nullptr, true));
     FL_CU(cudaMemcpyAsync(nx.data(), g->d_next, n * 4ull, cudaMemcpyDeviceToHost, g->stream));
     int h[kNumFlags];
     FL_TRY(sync_status(g, h));
