@@ -201,7 +201,10 @@ __device__ __forceinline__ void block_flag(int* flags, int slot, bool pred) {
 }
 
 // `0.0 + x` exactly as IEEE evaluates it: x itself, except that -0.0 becomes +0.0.
-__device__ __forceinline__ double plus_zero(double x) { return x == 0.0 ? 0.0 : x; }
+// Compared on the bits: an f64 comparison takes the f64 pipe.
+__device__ __forceinline__ double plus_zero(double x) {
+    return ((unsigned long long)__double_as_longlong(x) << 1) == 0 ? 0.0 : x;
+}
 
 // Nanosecond wall clock shared by all SMs (instrumentation).
 __device__ __forceinline__ uint64_t global_ns() {

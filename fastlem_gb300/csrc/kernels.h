@@ -13,13 +13,13 @@ enum KClass {
     kcNoise = 0,      // initial elevations
     kcReceivers,      // steepest-descent receivers
     kcLakes,          // basin labels + lake re-routing
-    kcBasinBuild,     // donor counts, leaves, skeleton collection / layout / preparation
+    kcBasinBuild,     // tiles bottom-up, first frontier, skeleton collection / layout / preparation
     kcKahn,           // bottom-up Kahn rounds (drainage area)
     kcSkelRank,       // pointer jumping over the skeleton
     kcSkelUp,         // skeleton chains bottom-up (drainage area)
     kcW,              // 1 / (k sqrt(A)) * len
     kcSkelDown,       // skeleton chains top-down (response time, elevation)
-    kcLowDown,        // Kahn rounds top-down (response time, elevation)
+    kcLowDown,        // Kahn rounds and tiles top-down (response time, elevation)
     kcMisc,
     kcResident,       // whole solves of resident terrains
     kcCount
@@ -77,7 +77,7 @@ inline unsigned sized_grid(bool sized, unsigned full, uint64_t units, uint64_t p
 
 // Device-side bookkeeping words of one basin pass (uint32 slots of BasinArgs::meta).
 enum Meta {
-    kMetaLeaves = 0,   // number of leaves (Kahn round 0)
+    kMetaLeaves = 0,   // sites of Kahn round 0: outside the tiles, all donors in tiles
     kMetaCnt0,         // rotating append counters of the Kahn rounds
     kMetaCnt1,
     kMetaCnt2,
@@ -152,7 +152,7 @@ struct BasinArgs {
     double* w_area;            // the A and receiver distance each w was computed from
     double* w_dist;
     bool w_valid;              // w / w_area / w_dist hold the previous pass's values
-    bool all_records;          // every site's record is read afterwards (else leaves skip it)
+    bool all_records;          // every site's record is read afterwards (else the tiles' skip it)
     double* elev;
     uint32_t* pending;
     uint32_t* hgt;
@@ -211,6 +211,7 @@ struct BasinArgs {
     uint32_t* tokslot;      // per donor-list entry: the slot whose list it is
     uint32_t* pend;         // per layout slot: chain bottoms still to push into its list
     uint32_t tok_cap;
+    bool tiles;             // the graph's rows are mutual and name no site twice
     uint64_t* push_to;      // per site: (stamp << 32) | tokval index its chain bottom fills
     int* bu_done;
     int* td_need;

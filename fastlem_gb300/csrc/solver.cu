@@ -493,6 +493,7 @@ struct fl_graph {
     // whole solves in one launch (resident.cu): the terrains' parts, in one device block
     // of ticket, barrier words (zeroed per launch), progress, terrains and slots
     bool resident = false;
+    bool simple = false;         // rows mutual, no site named twice (check_resident)
     bool res_slope = false;              // the plan has room for slope limits
     uint32_t largest = 0;                // sites of the largest terrain
     uint32_t res_cap = 0, res_slots = 0, res_blocks = 0;
@@ -1314,6 +1315,7 @@ int enqueue_basin_pass(fl_graph* g, bool all_records = false) {
     a.tokslot = g->d_tokslot;
     a.pend = g->d_pend;
     a.tok_cap = g->tok_cap;
+    a.tiles = g->simple;
     a.push_to = g->d_push;
     a.bu_done = g->d_bu_done;
     a.td_need = g->d_td_need;
@@ -1420,21 +1422,20 @@ struct ResidentLayout {
     }
 };
 
-// Whether every terrain's graph is one the resident solve takes (at set-up; the model's
+// Whether every terrain's graph is one the tiles and the resident solve take (at set-up; the model's
 // buffers are ready).
 int check_resident(fl_graph* g) {
     for (uint32_t t = 0; t < g->terrains; ++t)
         g->largest = std::max(g->largest, g->site_off[t + 1] - g->site_off[t]);
-    g->resident = g->largest <= (uint64_t)fl::resident_blocks() * fl::resident_cap(false) &&
-                  g->n < 0x80000000u;
-    if (!g->resident) return FL_OK;
+    if (g->n >= 0x80000000u) return FL_OK;
     FL_CU(cudaMemsetAsync(g->d_flags, 0, sizeof(int), g->stream));
     fl::launch_check_simple(g->stream, g->n, g->d_row, g->d_col, g->d_flags);
     FL_CU(cudaGetLastError());
     FL_CU(cudaMemcpyAsync(g->h_status, g->d_flags, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
     FL_CU(cudaMemsetAsync(g->d_flags, 0, sizeof(int), g->stream));
     FL_CU(cudaStreamSynchronize(g->stream));
-    g->resident = g->h_status[0] == 0;
+    g->simple = g->h_status[0] == 0;
+    g->resident = g->simple && g->largest <= (uint64_t)fl::resident_blocks() * fl::resident_cap(false);
     return FL_OK;
 }
 
@@ -1481,9 +1482,10 @@ int plan_resident(fl_graph* g) {
 // (about 0.3 us a site of the longest river and direction), the staged pass folds whole
 // chains but pays some 400 us of launches, barriers and skeleton building an iteration.
 // Measured without slope limits (32 iterations, staged / resident, ms): 10,000 sites 10.6 /
-// 2.3, 100,000 16.8 / 7.0, 200,000 19.0 / 13.6, 262,000 19.9 / 15.3, 400,000 22.5 / 16.4,
-// 450,000 25.5 / 36.3, 600,000 25.7 / 35.3.  With slope limits the staged walk is site by
-// site too: 100,000 29.5 / 10.5, 600,000 102 / 53.
+// 2.3, 150,000 16.5 / 11.6, 200,000 17.2 / 13.7, 230,000 17.4 / 17.2, 262,000 17.7 / 14.9,
+// 400,000 20.3 / 16.5, 450,000 25.5 / 36.3, 600,000 25.7 / 35.3 (the last two and the first before
+// the tiles).  With slope limits the staged walk is site by site too: 100,000 29.5 / 10.5,
+// 600,000 102 / 53.
 constexpr uint32_t kResidentLargest = 262144, kResidentLargestSlope = 786432;
 
 // Whether generate() takes the resident solve: a tuning override of the staged pass's
