@@ -5,15 +5,17 @@
 For each size class -- single terrains of about 64k, 256k, 1M, 4M and 16M sites (the
 16M benchmark terrain's generator at reduced scale: uniform sites, outlets on the left
 and bottom borders, value-noise erodibility) and one packed batch of terrains of uneven
-size -- it times generate() with set_max_iteration(8) (device time of the iteration
-loop, after two warm-up solves) while varying, one knob at a time:
+size -- it times generate() with set_max_iteration(32) (device time of the iteration
+loop, after two warm-up solves; a solve's first iterations are unlike the hundreds that
+follow) while varying, one knob at a time:
   kahn_min_width  where the Kahn rounds stop and the skeleton chain walks take over (the
                   round-versus-chain switch): the default rule n / 512 clamped to
                   [8192, 65536], times 1/16, 1/8, 1/4, 1/2 and 2;
   sized_grids     cooperative grids cut to the model's size, or the whole GPU;
   low_ilp         sites in flight per thread in the top-down Kahn rounds (1, 2, 4);
   walk_per_sm     chain walker blocks per SM (all that fit, 4, 2).
-Each knob keeps the best value found before the next is tried.  The results go to a
+Each knob keeps the best value found before the next is tried; a value replaces another for
+a gain of 1 % or more.  The results go to a
 JSON schedule (per class: the knobs, the time with the library defaults and with the
 chosen knobs, every trial); the library's compiled-in schedule is set from it.  Every
 shape gives the same bits (tests/test_gpu_tuning.py), so the sweep changes speed only.
@@ -95,7 +97,7 @@ def sweep(timer, n, log):
     def tryit(**kw):
         k = knobs(**kw)
         ms = run(k["kahn_min_width"], k["low_ilp"], k["walk_per_sm"], k["sized_grids"])
-        if ms < best["ms_per_iteration"]:
+        if ms < 0.99 * best["ms_per_iteration"]:      # a smaller gain is noise
             best.update(k, ms_per_iteration=ms)
 
     for f in (0.0625, 0.125, 0.25, 0.5, 2.0):
@@ -111,7 +113,7 @@ def sweep(timer, n, log):
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--out", default=os.path.join(HERE, "schedule.json"))
-    ap.add_argument("--iters", type=int, default=8)
+    ap.add_argument("--iters", type=int, default=32)
     ap.add_argument("--reps", type=int, default=2)
     ap.add_argument("--quick", action="store_true", help="sizes up to 1M only")
     args = ap.parse_args()

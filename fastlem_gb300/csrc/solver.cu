@@ -376,12 +376,12 @@ Tuning& tuning() {
 const std::vector<ScheduleEntry>& schedule() {
     static const std::vector<ScheduleEntry> s = {
         // max_sites, packed, {low_ilp, walk_per_sm, kahn_min_width}
-        {0x20000u, false, {4, 2, 512, false}},
-        {0x80000u, false, {4, 0, 1024, true}},
-        {0x200000u, false, {4, 0, 2048, true}},
-        {0x7d0000u, false, {4, 0, 4096, true}},
-        {0xffffffffu, false, {4, 4, 0, true}},
-        {0xffffffffu, true, {2, 0, 0, true}},
+        {0x20000u, false, {4, 0, 0, false}},
+        {0x80000u, false, {4, 0, 4096, false}},
+        {0x200000u, false, {4, 0, 4096, true}},
+        {0x7d0000u, false, {4, 0, 16384, true}},
+        {0xffffffffu, false, {4, 0, 0, false}},
+        {0xffffffffu, true, {4, 0, 0, false}},
     };
     return s;
 }
