@@ -193,22 +193,10 @@ def peak_hbm():
 # so the 1M config's launch (8th iteration of a generate(), --set full) is scaled by
 # the units (traffic grows with them).
 NCU_TRAFFIC = {
-    # 56.76 MB over the 939,485 Kahn-region sites (1,000,000 - 60,515 skeleton sites)
-    "kahn_rounds": (56.763e6 / 939_485, "kahn_sites",
-                    "ncu dram__bytes_read+write of one k_kahn launch on the 1M config "
-                    "(8th iteration), scaled by Kahn-region sites"),
     # 3.064 MB over 60,515 skeleton sites
     "skeleton_up": (3.064e6 / 60_515, "skeleton_sites",
                     "ncu dram__bytes_read+write of one k_s_bottom_up launch on the 1M config "
                     "(8th iteration), scaled by skeleton sites"),
-    # 113.38 MB over 1,000,000 sites
-    "receivers": (113.38e6 / 1_000_000, "sites",
-                  "ncu dram__bytes_read+write of one k_receivers launch on the 1M config "
-                  "(8th iteration), scaled by sites"),
-    # 52.40 MB over the 939,485 Kahn-region sites
-    "rounds_down": (52.40e6 / 939_485, "kahn_sites",
-                    "ncu dram__bytes_read+write of one k_low_top_down launch on the 1M config "
-                    "(8th iteration), scaled by Kahn-region sites"),
     # 39.41 MB over 1,000,000 sites
     "response_w": (39.41e6 / 1_000_000, "sites",
                    "ncu dram__bytes_read+write of one k_w launch on the 1M config "
@@ -220,8 +208,7 @@ def measured_traffic(kernel, basin, n):
     if kernel not in NCU_TRAFFIC:
         return None, "no ncu capture for this kernel"
     per, unit, src = NCU_TRAFFIC[kernel]
-    units = {"skeleton_sites": basin["skeleton_sites"], "sites": n,
-             "kahn_sites": n - basin["skeleton_sites"]}[unit]
+    units = {"skeleton_sites": basin["skeleton_sites"], "sites": n}[unit]
     return per * units, src
 
 

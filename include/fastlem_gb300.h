@@ -220,7 +220,8 @@ int fl_select_device(int device);
 int fl_graph_set_timing(fl_graph* g, int enable);
 void fl_graph_reset_stats(fl_graph* g);
 /* Blocking host synchronisations the model's calls made since the last reset: one per
- * iteration of generate(), one more in an iteration that computes the lake order. */
+ * staged iteration of generate() (one for all iterations of a resident solve), one more in
+ * an iteration that computes the lake order. */
 uint64_t fl_graph_host_syncs(const fl_graph* g);
 
 /* Launch shapes and switch points of the solve (no counterpart in the reference; the
@@ -260,15 +261,15 @@ uint32_t fl_num_kernel_classes(void);
 int fl_graph_kernel_stats(const fl_graph* g, uint32_t cls, const char** name, uint64_t* launches,
                           double* device_ms, double* bytes);
 
-/* Shape of the last basin pass (up to `cap` values): Kahn rounds run, leaves,
- * skeleton sites, skeleton chains, longest chain, skeleton sites needing the full
+/* Shape of the last staged basin pass (up to `cap` values; a resident solve leaves them as
+ * they were): Kahn rounds run, sites of the first round, skeleton sites, skeleton chains, longest chain, skeleton sites needing the full
  * pull while walking, bottom-up and top-down hand-off wait iterations; then the
  * slowest bottom-up chain's walk time (ns), SM cycles spent in its full pulls and
  * their number; the slowest top-down chain's walk time (ns), SM cycles waiting for
  * its parent and its length.  Durations are kept to 64 ns, cycles to 128. */
 int fl_graph_basin_stats(const fl_graph* g, uint64_t* out, uint32_t cap);
 
-/* Round structure of the last basin pass (instrumentation; no fastlem counterpart).
+/* Round structure of the last staged basin pass (instrumentation; no fastlem counterpart).
  * *rounds = Kahn rounds run (r); for k <= min(cap - 1, r): offsets[k] = first order
  * slot of Kahn round k, up_ns[k] = device clock (ns) when bottom-up round k started
  * (up_ns[r] = end), down_ns[k] = when the k-th top-down round started (highest Kahn
