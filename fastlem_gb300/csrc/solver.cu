@@ -1487,6 +1487,11 @@ int plan_resident(fl_graph* g) {
 // the tiles).  With slope limits the staged walk is site by site too: 100,000 29.5 / 10.5,
 // 600,000 102 / 53.
 constexpr uint32_t kResidentLargest = 262144, kResidentLargestSlope = 786432;
+// The most sites of all packed terrains together: a packed resident solve is bound by the
+// blocks' throughput, the staged one by its launches first.  Terrains of 47,000 sites, staged /
+// resident, ms an iteration: 1.5M sites 0.77 / 0.71, 3.0M 1.09 / 1.10, 4.5M 1.41 / 1.51, 9M 2.30 /
+// 2.89; with slope limits 3.0M 2.19 / 1.72, 4.5M 2.64 / 2.49, 6M 3.15 / 3.27.
+constexpr uint64_t kResidentTotal = 3145728, kResidentTotalSlope = 5242880;
 
 // Whether generate() takes the resident solve: a tuning override of the staged pass's
 // shapes asks for that pass.
@@ -1495,7 +1500,8 @@ bool use_resident(const fl_graph* g) {
     return g->resident && g->largest <= (uint64_t)fl::resident_blocks() * fl::resident_cap(g->slope) &&
            t.resident != 0 && t.low_ilp < 0 && t.walk_per_sm < 0 &&
            t.kahn_min_width < 0 && t.sized_grids < 0 &&
-           (t.resident == 1 || g->largest <= (g->slope ? kResidentLargestSlope : kResidentLargest));
+           (t.resident == 1 || (g->largest <= (g->slope ? kResidentLargestSlope : kResidentLargest) &&
+                                g->n <= (g->slope ? kResidentTotalSlope : kResidentTotal)));
 }
 
 enum ResidentEnd {
