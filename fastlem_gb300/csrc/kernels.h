@@ -336,7 +336,6 @@ struct ResidentArgs {
     uint32_t *lab, *lab2;
     unsigned long long* best;
     double *xarea, *xtime, *xelev;   // exchange slots: two, four and two values per site
-    double* troot;
     const ResidentTerrain* terrains;
     const uint32_t* slot_terrain;
     ResidentCtrl* ctrl;

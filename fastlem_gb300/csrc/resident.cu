@@ -32,7 +32,10 @@
 // Values published across blocks use two slots per site, by the iteration's parity: a slot
 // is set back to the pending marker one iteration later, when its readers have passed a
 // barrier, so the publishing store is itself the flag (a time travels with its basin's root
-// as one 16-byte value) and an iteration needs two barriers.  Every wait is bounded.
+// as one 16-byte value) and an iteration needs two barriers.  That a value has arrived says
+// nothing about any other address -- the stores and loads are relaxed, and values go on
+// through third blocks -- so whoever needs a root's time and elevation polls the root's own
+// slots; in practice they are there at the first look.  Every wait is bounded.
 //
 // One launch takes many terrains (packed models): blocks take (terrain, part) slots in
 // order, largest terrains first, and a terrain starts when its last part is taken.  Only
@@ -68,8 +71,6 @@ __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long l
     asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
-// An ordering fence without the sequential consistency of __threadfence.
-__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ uint64_t bits(double x) { return (uint64_t)__double_as_longlong(x); }
 __device__ __forceinline__ double from_bits(uint64_t b) { return __longlong_as_double((long long)b); }
 // NaN payloads are not published (integer test: an f64 comparison takes 109 cycles)
@@ -85,11 +86,10 @@ __device__ __forceinline__ void st_relaxed128(void* p, uint64_t lo, uint64_t hi)
     asm volatile("{.reg .b128 t; mov.b128 t, {%1, %2}; st.relaxed.gpu.global.b128 [%0], t;}" ::"l"(p), "l"(lo), "l"(hi) : "memory");
 }
 // Exchange slots of site g (by iteration parity): area; response time with the basin's root,
-// as one 16-byte value; limited elevation.  And a root's own response time.
+// as one 16-byte value; limited elevation, or a root's elevation.
 __device__ __forceinline__ double* area_slot(const ResidentArgs& a, uint32_t g, uint32_t par) { return a.xarea + 2ull * g + par; }
 __device__ __forceinline__ double* time_slot(const ResidentArgs& a, uint32_t g, uint32_t par) { return a.xtime + 4ull * g + 2 * par; }
 __device__ __forceinline__ double* elev_slot(const ResidentArgs& a, uint32_t g, uint32_t par) { return a.xelev + 2ull * g + par; }
-__device__ __forceinline__ double* root_time(const ResidentArgs& a, uint32_t g) { return a.troot + g; }
 
 __device__ __forceinline__ void raise(ResidentCtrl* c, int code) { atomicCAS(&c->error, 0, code); }
 
@@ -556,8 +556,8 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
         const uint32_t g = lo + v;
         for (uint32_t par = 0; par < 2; ++par) {
             st_relaxed64(area_slot(a, g, par), kPendingBits);
-            st_relaxed64(time_slot(a, g, par), kPendingBits);
-            if (kSlope) st_relaxed64(elev_slot(a, g, par), kPendingBits);
+            st_relaxed128(time_slot(a, g, par), kPendingBits, 0);
+            st_relaxed64(elev_slot(a, g, par), kPendingBits);
         }
         sts32(bk.word(v), 0);
     }
@@ -581,9 +581,9 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
             // last iteration's published values have been read: their slots are free
             const uint32_t was = lds32(bk.word(v));
             if (was & kFar) st_relaxed64(area_slot(a, g, par ^ 1u), kPendingBits);
-            if (was & kFarDonor) {
-                st_relaxed64(time_slot(a, g, par ^ 1u), kPendingBits);
-                if (kSlope) st_relaxed64(elev_slot(a, g, par ^ 1u), kPendingBits);
+            if (was & (kFarDonor | kRoot)) {
+                st_relaxed128(time_slot(a, g, par ^ 1u), kPendingBits, 0);
+                if (kSlope || (was & kRoot)) st_relaxed64(elev_slot(a, g, par ^ 1u), kPendingBits);
             }
             uint32_t slot = kNone;
             if (!__ldg(&a.outlet[g])) {
@@ -790,9 +790,10 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
             }
             const double t = plus_zero(plus_zero(wv));
             const bool out = __ldg(&a.outlet[g]) != 0;
+            double ne = __ldcg(&a.elev[g]);
             if (out) {
-                const double old_e = __ldcg(&a.elev[g]), dt = __dsub_rn(t, t);
-                double ne = __dadd_rn(old_e, __dmul_rn(__ldg(&a.u[g]), dt > 0.0 ? dt : 0.0));
+                const double old_e = ne, dt = __dsub_rn(t, t);
+                ne = __dadd_rn(old_e, __dmul_rn(__ldg(&a.u[g]), dt > 0.0 ? dt : 0.0));
                 if (kSlope) {
                     const double tn = __ldg(&a.tanms[g]), dist = __ldcg(&a.rlen[g]);
                     if (!isnan(tn) && __ddiv_rn(__dsub_rn(ne, old_e), dist) > tn)
@@ -803,10 +804,11 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
                 a.pair[g] = float_pair(ne);
             }
             const uint32_t root = out ? g : g | kNoOutlet;
-            *root_time(a, g) = t;              // before the time that leads here is published
             sts128(r, bits(t), (uint64_t)1 << 32 | root);
-            fence_gpu();       // ... on the whole GPU: other blocks read them once they have that time
-            if (w & kFarDonor) st_relaxed128(time_slot(a, g, par), published(t), root);
+            // for its donors in other blocks and for its basin's sites, wherever they are (an
+            // elevation is the result of an addition, so never the pending marker)
+            st_relaxed128(time_slot(a, g, par), published(t), root);
+            st_relaxed64(elev_slot(a, g, par), bits(ne));
         }
         __syncthreads();
         if (!settle_down<kSlope, true>(a, gr, bk, lo, S, par, nout)) {
@@ -814,13 +816,25 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
             break;
         }
         // ---- elevations
+        uint32_t spins = 0;
 #pragma unroll 1
         for (uint32_t u = tid; u < S; u += kT) {
             const uint32_t g = lo + u, rec = bk.rec(u), r = lds32(rec + fRoot);
             const bool is_root = (r & ~kNoOutlet) == g;
             double ne = 0.0;
             if (!(r & kNoOutlet) && !is_root) {
-                const double to = __ldcg(root_time(a, r)), eo = __ldcg(&a.elev[r]);
+                uint64_t tb, eb, root;
+                while (true) {
+                    ld_relaxed128(time_slot(a, r, par), tb, root);
+                    eb = ld_relaxed64(elev_slot(a, r, par));
+                    if (tb != kPendingBits && eb != kPendingBits) break;
+                    if (give_up(gr, spins)) {
+                        lost = true;
+                        break;
+                    }
+                }
+                if (lost) break;
+                const double to = from_bits(tb), eo = from_bits(eb);
                 const double dt = __dsub_rn(ldsd(rec), to);
                 ne = __dadd_rn(eo, __dmul_rn(__ldg(&a.u[g]), dt > 0.0 ? dt : 0.0));
                 if (!kSlope) {
@@ -836,12 +850,14 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
                 // cannot stand in for the quotient
                 const double tn = __ldg(&a.tanms[g]), dist = __ldcg(&a.rlen[g]), rise = __dmul_rn(tn, dist);
                 stsd(bk.lim + 8 * u, tn > 1e-200 && dist > 0.0 && rise > 1e-200 && rise < 1e200 && !(r & kNoOutlet) ? rise : -1.0);
-                if (is_root && (lds32(bk.word(u)) & kFarDonor)) st_relaxed64(elev_slot(a, g, par), published(ne));
                 sts128(rec, bits(ne), (uint64_t)(is_root ? 2 : 1) << 32 | r);
             }
         }
+        if (__syncthreads_or(lost)) {
+            gr.ok = false;
+            break;
+        }
         if (kSlope) {
-            __syncthreads();
             if (!settle_down<kSlope, false>(a, gr, bk, lo, S, par, nout)) {
                 gr.ok = false;
                 break;

@@ -1561,7 +1561,6 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     a.xtime = reinterpret_cast<double*>(g->d_trec);
     a.xarea = reinterpret_cast<double*>(g->d_rec);
     a.xelev = a.xarea + 2ull * g->n;
-    a.troot = g->d_el;
     a.terrains = reinterpret_cast<const ResidentTerrain*>(d + lay.terrains);
     a.slot_terrain = reinterpret_cast<const uint32_t*>(d + lay.slots);
     a.ctrl = reinterpret_cast<ResidentCtrl*>(d + lay.ctrl);
