@@ -322,14 +322,17 @@ __global__ void k_fill_f64(uint32_t n, double* __restrict__ a, const double* __r
     if (i < n) a[i] = src ? src[i] : 0.0;
 }
 
-// Packed terrains: a terrain whose elevations did not change in iteration `iter`
-// (1-based) would have stopped there alone; its first such iteration is recorded, and
-// the per-terrain "changed" words are cleared for the next iteration.
+// Packed terrains: a terrain whose elevations did not change in an iteration would have
+// stopped there alone; its first such iteration is recorded, or the limit when it comes
+// first, and the per-terrain "changed" words are cleared for the next iteration.  step
+// (1-based) counts the staged iterations, start those that the terrain had before them.
 __global__ void k_terrain_iters(uint32_t terrains, int* __restrict__ tchg,
-                                uint32_t* __restrict__ titer, uint32_t iter) {
+                                uint32_t* __restrict__ titer, const uint32_t* __restrict__ start,
+                                uint32_t step, uint32_t limit) {
     uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= terrains) return;
-    if (!tchg[t] && titer[t] == 0) titer[t] = iter;
+    const uint32_t iter = start[t] + step;
+    if ((!tchg[t] || iter >= limit) && titer[t] == 0) titer[t] = iter;
     tchg[t] = 0;
 }
 
@@ -443,7 +446,9 @@ struct fl_graph {
     uint32_t* d_noise_idx = nullptr;   // device site -> its sample (index within its terrain)
     uint32_t* d_tid = nullptr;
     int* d_tchg = nullptr;
-    uint32_t* d_titer = nullptr;   // per terrain: first iteration without a change (0: none yet)
+    // per terrain: first iteration without a change, or the last one (0: none yet), then the
+    // iterations done before the staged ones (k_terrain_iters)
+    uint32_t* d_titer = nullptr;
     // page-locked copy of the status words and basin-pass bookkeeping, read once per
     // iteration
     int* h_status = nullptr;
@@ -498,6 +503,7 @@ struct fl_graph {
     uint32_t largest = 0;                // sites of the largest terrain
     uint32_t res_cap = 0, res_slots = 0, res_blocks = 0;
     unsigned char* d_resident = nullptr;
+    std::vector<uint8_t> res_never;      // terrains that the resident solve has no room for
     // instrumentation: launches / algorithmic bytes always, device time when enabled
     bool timing = false;
     uint64_t k_launches[kcCount] = {};
@@ -1504,21 +1510,46 @@ bool use_resident(const fl_graph* g) {
                                 g->n <= (g->slope ? kResidentTotalSlope : kResidentTotal)));
 }
 
-enum ResidentEnd {
-    kResidentDone,       // every terrain settled or at the limit
-    kResidentNoRoom,     // a block met more far donors than it has room for: the model keeps
-                         // to the staged pass, and d_elev is to be set up again
-    kResidentSlow        // long rivers: the staged pass is to go on from d_elev (one terrain)
-};
-// The iterations of every terrain from the initial elevations in d_elev; iters[t]:
-// iterations of terrain t.
+// Initial elevations of the device sites [lo, lo + m); the noise is in d_w.
+int initial_elevations(fl_graph* g, uint32_t lo, uint32_t m) {
+    FL_LAUNCH(g, kcNoise, 28.0 * m,
+              k_initial_elevation<<<blocks_for(m), kThreads, 0, g->stream>>>(
+                  m, (g->d_noise_idx ? g->d_noise_idx : g->d_perm) + lo, g->d_base + lo, g->d_w,
+                  g->d_elev + lo, g->d_pair + lo));
+    FL_CU(cudaGetLastError());
+    return FL_OK;
+}
+
+// Every terrain draws its own StdRng::seed_from_u64(0) stream, sample i for its site i.
+int noise(fl_graph* g) {
+    FL_LAUNCH(g, kcNoise, 8.0 * g->noise_n,
+              k_noise<<<blocks_for((g->noise_n + 7) / 8), kThreads, 0, g->stream>>>(g->noise_n, g->d_w));
+    g->w_valid = false;
+    FL_CU(cudaGetLastError());
+    return FL_OK;
+}
+
+// The iterations of every terrain from the initial elevations in d_elev.  settled[t]: the
+// iterations of terrain t, or 0 where the staged iterations are to go on from d_elev after
+// start[t] iterations: 0 for a terrain that the kernel raised an error on, which starts again
+// (its error, if the staged pass meets it too, is that pass's to report).  One that met more
+// far donors than a block has room for is not tried again.
 int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t limit,
-                   std::vector<uint32_t>& iters, ResidentEnd* end) {
+                   std::vector<uint32_t>& settled, std::vector<uint32_t>& start) {
     const uint32_t k = g->terrains;
     FL_TRY(plan_resident(g));
     const ResidentLayout lay(k, g->res_slots);
     unsigned char* d = g->d_resident;
-    FL_CU(cudaMemsetAsync(d + lay.ctrl, 0, sizeof(ResidentCtrl) * k, g->stream));
+    std::vector<ResidentCtrl> ctrl(k);
+    g->res_never.resize(k);
+    bool more = false;
+    for (uint32_t t = 0; t < k; ++t) {
+        ctrl[t].done = g->res_never[t];
+        more |= !ctrl[t].done;
+    }
+    if (!more) return FL_OK;
+    FL_CU(cudaMemcpyAsync(d + lay.ctrl, ctrl.data(), sizeof(ResidentCtrl) * k, cudaMemcpyHostToDevice,
+                          g->stream));
     int h[kNumFlags];
     if (!g->rank_uploaded) {                  // the first iteration's lakes
         FL_TRY(clear_flags(g));
@@ -1567,8 +1598,8 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     a.bars = reinterpret_cast<unsigned long long*>(d + lay.bars);
     a.ticket = reinterpret_cast<uint32_t*>(d + lay.ticket);
     g->w_valid = false;
-    std::vector<ResidentCtrl> ctrl(k);
-    bool more = true;
+    std::vector<uint8_t> ended(k), again(k);
+    for (uint32_t t = 0; t < k; ++t) ended[t] = ctrl[t].done != 0;
     while (more) {
         FL_CU(cudaMemsetAsync(d, 0, lay.ctrl, g->stream));
         a.rank_ready = g->rank_uploaded;
@@ -1585,25 +1616,35 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
         more = false;
         bool need_rank = false;
         for (uint32_t t = 0; t < k; ++t) {
-            if (ctrl[t].error == kErrCapacity) {
-                *end = kResidentNoRoom;
-                g->resident = false;
-                return FL_OK;
+            ResidentCtrl& c = ctrl[t];
+            if (ended[t]) continue;
+            need_rank |= c.need_rank != 0;
+            c.need_rank = 0;
+            if (c.error != 0) {
+                again[t] = 1;
+                if (c.error == kErrCapacity) g->res_never[t] = 1;
+            } else if (c.slow) {
+                start[t] = c.iters;
+            } else if (c.done) {
+                settled[t] = c.iters;
+            } else {
+                more = true;
+                continue;
             }
-            h[kError] = ctrl[t].error;
-            FL_TRY(device_error(h));
-            if (ctrl[t].slow) *end = kResidentSlow;
-            more |= !ctrl[t].done && !ctrl[t].slow;
-            need_rank |= ctrl[t].need_rank != 0;
-            iters[t] = ctrl[t].iters;
+            ended[t] = 1;
+            c.done = 1;
         }
-        if (need_rank) {
-            FL_TRY(set_outlets(g, outlets, true));
-            for (uint32_t t = 0; t < k; ++t) ctrl[t].need_rank = 0;
+        if (need_rank) FL_TRY(set_outlets(g, outlets, true));
+        if (more)
             FL_CU(cudaMemcpyAsync(d + lay.ctrl, ctrl.data(), sizeof(ResidentCtrl) * k, cudaMemcpyHostToDevice,
                                   g->stream));
-            FL_CU(cudaStreamSynchronize(g->stream));
-        }
+    }
+    bool drawn = false;
+    for (uint32_t t = 0; t < k; ++t) {
+        if (!again[t]) continue;
+        if (!drawn) FL_TRY(noise(g));
+        drawn = true;
+        FL_TRY(initial_elevations(g, g->site_off[t], g->site_off[t + 1] - g->site_off[t]));
     }
     return FL_OK;
 }
@@ -1629,49 +1670,41 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
     FL_TRY(set_outlets(g, outlets, false));
     // all status words, including the grid barrier's, start from zero
     FL_CU(cudaMemsetAsync(g->d_flags, 0, kNumFlags * sizeof(int), g->stream));
-    // every terrain draws its own StdRng::seed_from_u64(0) stream, sample i for its site i
-    auto initial_elevations = [&]() -> int {
-        FL_LAUNCH(g, kcNoise, 8.0 * g->noise_n,
-                  k_noise<<<blocks_for((g->noise_n + 7) / 8), kThreads, 0, g->stream>>>(g->noise_n, g->d_w));
-        g->w_valid = false;
-        FL_LAUNCH(g, kcNoise, 28.0 * n,
-                  k_initial_elevation<<<blocks_for(n), kThreads, 0, g->stream>>>(
-                      n, g->d_noise_idx ? g->d_noise_idx : g->d_perm, g->d_base, g->d_w, g->d_elev, g->d_pair));
-        FL_CU(cudaGetLastError());
-        return FL_OK;
-    };
-    FL_TRY(initial_elevations());
+    FL_TRY(noise(g));
+    FL_TRY(initial_elevations(g, 0, n));
     if (max_iter > 0xffffffffll) max_iter = 0xffffffffll;
     uint64_t limit = max_iter < 0 ? 0xffffffffull : (uint64_t)max_iter;
     uint32_t iters = 0;
-    uint64_t done = 0;                                // iterations of the resident solve
+    // iterations of the terrains that the resident solve settled, and of the others in it
+    std::vector<uint32_t> settled_at(g->terrains, 0), start(g->terrains, 0);
+    const bool resident = limit > 0 && use_resident(g);
     FL_CU(cudaEventRecord(g->ev0, g->stream));
-    if (limit > 0 && use_resident(g)) {
-        std::vector<uint32_t> each(g->terrains);
-        ResidentEnd end = kResidentDone;
-        FL_TRY(resident_solve(g, outlets, limit, each, &end));
-        if (end == kResidentDone) {
-            for (uint32_t t = 0; t < g->terrains; ++t) {
-                iters = std::max(iters, each[t]);
-                if (terrain_iters) terrain_iters[t] = each[t];
-            }
+    if (resident) {
+        FL_TRY(resident_solve(g, outlets, limit, settled_at, start));
+        if (std::find(settled_at.begin(), settled_at.end(), 0u) == settled_at.end()) {
+            iters = *std::max_element(settled_at.begin(), settled_at.end());
+            if (terrain_iters) std::copy(settled_at.begin(), settled_at.end(), terrain_iters);
             return finish_generate(g, out_elev, iters, out_iters, loop_ms, total_ms, t_start);
         }
-        if (end == kResidentNoRoom) FL_TRY(initial_elevations());
-        else done = each[0];
     }
+    // a pack's staged iterations count from those of the terrain that has the fewest
+    uint64_t done = limit;
+    for (uint32_t t = 0; t < g->terrains; ++t)
+        if (!settled_at[t]) done = std::min<uint64_t>(done, start[t]);
     // previous-iteration drainage areas steer the skeleton's chain choice; start from
     // the cell areas
     FL_LAUNCH(g, kcMisc, 16.0 * n,
               k_fill_f64<<<blocks_for(n), kThreads, 0, g->stream>>>(n, g->d_A, g->d_area));
     FL_CU(cudaGetLastError());
-    if (done == 0) FL_CU(cudaEventRecord(g->ev0, g->stream));   // the loop's time starts here
+    if (!resident) FL_CU(cudaEventRecord(g->ev0, g->stream));   // the loop's time starts here
     g->passes = 0;
     // a terrain alone stops at its first iteration without a change; packed with others
     // it keeps iterating at a fixed point, so its count is that first unchanged iteration
     if (g->d_titer) {
         FL_CU(cudaMemsetAsync(g->d_tchg, 0, g->terrains * sizeof(int), g->stream));
-        FL_CU(cudaMemsetAsync(g->d_titer, 0, g->terrains * sizeof(uint32_t), g->stream));
+        for (uint32_t v : start) settled_at.push_back(v - std::min(v, (uint32_t)done));
+        FL_CU(cudaMemcpyAsync(g->d_titer, settled_at.data(), settled_at.size() * 4ull, cudaMemcpyHostToDevice,
+                              g->stream));
     }
     // One host synchronisation per iteration, on the status of the iteration before:
     // whether an elevation changed (the loop's exit, generator.rs:207-209) and any
@@ -1707,7 +1740,8 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
         FL_TRY(enqueue_basin_pass(g));
         if (g->d_titer) {
             k_terrain_iters<<<blocks_for(g->terrains), kThreads, 0, g->stream>>>(
-                g->terrains, g->d_tchg, g->d_titer, (uint32_t)(it + 1));
+                g->terrains, g->d_tchg, g->d_titer, g->d_titer + g->terrains, (uint32_t)(it + 1),
+                (uint32_t)limit);
             FL_CU(cudaGetLastError());
         }
         FL_TRY(enqueue_status(g, (int)(it & 1)));
@@ -1723,16 +1757,17 @@ int generate_impl(fl_graph* g, uint32_t n_params, HostCols<const double> base,
         if (int rc = take_status(g, (int)((it - 1) & 1), h)) return drained(rc);
         iters = (uint32_t)it;
     }
-    if (terrain_iters) {
-        if (g->d_titer) {
-            FL_CU(cudaMemcpyAsync(terrain_iters, g->d_titer, g->terrains * sizeof(uint32_t),
-                                  cudaMemcpyDeviceToHost, g->stream));
-            FL_CU(cudaStreamSynchronize(g->stream));
-            for (uint32_t t = 0; t < g->terrains; ++t)
-                if (!terrain_iters[t]) terrain_iters[t] = iters;
-        } else {
-            terrain_iters[0] = iters;
+    if (g->d_titer) {
+        FL_CU(cudaMemcpyAsync(start.data(), g->d_titer, g->terrains * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                              g->stream));
+        FL_CU(cudaStreamSynchronize(g->stream));
+        for (uint32_t t = 0; t < g->terrains; ++t) {
+            const uint32_t each = start[t] ? start[t] : iters;
+            if (terrain_iters) terrain_iters[t] = each;
+            if (resident) iters = std::max(iters, each);
         }
+    } else if (terrain_iters) {
+        terrain_iters[0] = iters;
     }
     return finish_generate(g, out_elev, iters, out_iters, loop_ms, total_ms, t_start);
 }
@@ -1850,7 +1885,7 @@ int create_graph(uint32_t n, const uint32_t* row_ptr, const uint32_t* col, const
         return fail(rc);
     if (k_terr > 1 &&
         ((rc = dalloc(&g->d_noise_idx, n)) || (rc = dalloc(&g->d_tid, n)) ||
-         (rc = dalloc(&g->d_tchg, k_terr)) || (rc = dalloc(&g->d_titer, k_terr))))
+         (rc = dalloc(&g->d_tchg, k_terr)) || (rc = dalloc(&g->d_titer, 2ull * k_terr))))
         return fail(rc);
     // upload, check and relabel on the device
     fl::GraphInput gi{n, nnz, row_ptr, col, len, area, (xs && ys) ? xs : nullptr,
