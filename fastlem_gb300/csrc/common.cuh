@@ -31,6 +31,7 @@ enum DeviceError {
     kErrBarrier = 2,      // a grid barrier wait ran out
     kErrWait = 3,         // a chain hand-off wait ran out
     kErrCapacity = 4,     // a fixed-size table overflowed
+    kErrLate = 5,         // the resident solve: its first iteration is past its time
 };
 
 // Spin limits: a wait that exceeds them reports an error instead of hanging.

@@ -304,6 +304,7 @@ constexpr size_t kResidentSmem = 226 * 1024; // shared memory of a block, at mos
 // 87.4 / 170.
 constexpr uint32_t kResidentPart = 448;
 constexpr uint32_t kResidentMaxRow = 64;     // longest adjacency row taken
+constexpr uint32_t kSlowPoints = 4;
 // A terrain's device sites [lo, lo + n), cut into `parts` block ranges; slot0: its first
 // (terrain, part) slot.
 struct ResidentTerrain {
@@ -315,13 +316,16 @@ struct ResidentCtrl {
     uint32_t done;         // settled, or at the limit
     int error;             // kErr*
     uint32_t need_rank;    // stopped: an iteration found lakes before the lake order was there
-    uint32_t slow;         // stopped: iterations over the time limit
-    uint32_t pad[3];
+    uint32_t slow;         // time rule (ResidentArgs::slow_ns): the last iterations' points
+    uint32_t left;         // stopped: long rivers, the staged pass is to go on
+    uint32_t pad[2];
 };
 struct ResidentArgs {
     uint32_t n, cap, slots, chunk;   // chunk: most iterations of a terrain per launch
     uint32_t limit;
-    uint64_t slow_ns;                // stop after four iterations in a row over this; 0: never
+    // an iteration over this counts one point and one over twice this kSlowPoints, one that
+    // is not clears them, and kSlowPoints end the terrain's solve; 0: no rule
+    uint64_t slow_ns;
     bool rank_ready;
     const uint32_t *row, *col;
     const double* len;

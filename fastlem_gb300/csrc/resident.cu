@@ -142,12 +142,22 @@ __device__ __noinline__ bool group_barrier(Group& gr, bool pred, bool ask = fals
     return any;
 }
 
+// When the block's waits of the iteration are to be given up (global_ns; shared).
+__device__ __forceinline__ unsigned long long& wait_until() {
+    __shared__ unsigned long long ns;
+    return ns;
+}
+constexpr unsigned long long kNoTime = ~0ull;
+
 __device__ __forceinline__ bool give_up(Group& gr, uint32_t& spins) {
     if (++spins > kSpinLimit) {
         raise(gr.ctrl, kErrWait);
         return true;
     }
-    return (spins & 255) == 0 && ld_acquire(&gr.ctrl->error) != 0;
+    if ((spins & 255) != 0) return false;
+    const unsigned long long until = wait_until();
+    if (until != kNoTime && global_ns() > until) raise(gr.ctrl, kErrLate);
+    return ld_acquire(&gr.ctrl->error) != 0;
 }
 
 // The reference's scan of site g's row: its slot, or kNone.
@@ -564,7 +574,7 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
     if (tid == 0) stsd(bk.rec(bk.none), -0.0);
     group_barrier(gr, false);
 
-    uint32_t slow = 0;                        // iterations in a row over the time limit
+    uint32_t slow = 0;                        // the time rule's points
     while (gr.ok && it < stop) {
         const uint32_t par = it & 1u;
         const uint64_t t0 = a.slow_ns && gr.part == 0 && tid == 0 ? global_ns() : 0;
@@ -669,6 +679,9 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
                 if (out && ot < kEdges) sts16(bk.out + 2 * ot, v);
             }
         }
+        // the first iteration's rivers are as long as any: past the time for which the rule
+        // ends a solve at once, it is dropped on the way (all its waits are behind this point)
+        if (tid == 0) wait_until() = a.slow_ns && it == 0 ? global_ns() + 2 * a.slow_ns : kNoTime;
         __syncthreads();
         const uint32_t nleaf = s_fin, nfar = s_far, nout = s_out;
         __syncthreads();                      // ... before the walks count on
@@ -873,19 +886,25 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
             }
         }
         ++it;
-        if (t0) slow = global_ns() - t0 > a.slow_ns ? slow + 1 : 0;
-        const bool more = group_barrier(gr, changed, slow >= 4);
+        if (t0) {
+            const uint64_t took = global_ns() - t0;
+            slow = took <= a.slow_ns ? 0 : slow + (took > 2 * a.slow_ns ? kSlowPoints : 1);
+        }
+        const bool more = group_barrier(gr, changed, slow >= kSlowPoints);
         if (!gr.ok) break;
         if (!more || it >= a.limit) {
             if (gr.part == 0 && tid == 0) ctrl->done = 1;
             break;
         }
         if (gr.stop) {                        // long rivers: the staged pass goes on
-            if (gr.part == 0 && tid == 0) ctrl->slow = 1;
+            if (gr.part == 0 && tid == 0) ctrl->left = 1;
             break;
         }
     }
-    if (gr.part == 0 && tid == 0) ctrl->iters = it;
+    if (gr.part == 0 && tid == 0) {
+        ctrl->iters = it;
+        ctrl->slow = slow;
+    }
 }
 
 template <bool kSlope>

@@ -503,7 +503,8 @@ struct fl_graph {
     uint32_t largest = 0;                // sites of the largest terrain
     uint32_t res_cap = 0, res_slots = 0, res_blocks = 0;
     unsigned char* d_resident = nullptr;
-    std::vector<uint8_t> res_never;      // terrains that the resident solve has no room for
+    // per terrain: solves under the time rule that it sits out, kNeverResident: all solves
+    std::vector<uint8_t> res_rest;
     // instrumentation: launches / algorithmic bytes always, device time when enabled
     bool timing = false;
     uint64_t k_launches[kcCount] = {};
@@ -1529,11 +1530,30 @@ int noise(fl_graph* g) {
     return FL_OK;
 }
 
+// A terrain whose rivers are long for the resident solve sits out the next kRestSolves solves
+// of its model: they take the staged iterations' time from the start, and what trying again
+// costs -- at most two staged iterations for the first, dropped one -- is shared by sixteen.
+// (Not for ever: its parameters, and with them its rivers, may be others by then, or the time
+// another stream's doing.)  One that met more far donors than a block has room for, or
+// another error, is not tried again.
+constexpr uint8_t kRestSolves = 15, kNeverResident = 255;
+
+// The time that a resident iteration may take (ResidentArgs::slow_ns): about what a staged
+// one takes -- 0.28 ms at 1,000 sites, 0.45 at 65,000, 0.55 at 262,000.  A pack's terrain runs
+// beside the others, so it pays to leave only past the sum of the resident iteration that goes
+// on without it and the staged one that it then needs, both of the whole pack: twice 0.77 ms
+// at 1.5M sites, 1.09 at 3.0M.  With slope limits the staged walk goes site by site as well,
+// 3.5 times as slow (a single file of 20,000 sites to convergence 65 ms against 18.2, of
+// 100,000 sites 320 against 91): no rule.
+uint64_t resident_slow_ns(const fl_graph* g) {
+    if (g->slope || fl::tuning().resident == 1) return 0;
+    return g->terrains == 1 ? 400000ull + g->n : 800000ull + g->n / 2;
+}
+
 // The iterations of every terrain from the initial elevations in d_elev.  settled[t]: the
 // iterations of terrain t, or 0 where the staged iterations are to go on from d_elev after
 // start[t] iterations: 0 for a terrain that the kernel raised an error on, which starts again
-// (its error, if the staged pass meets it too, is that pass's to report).  One that met more
-// far donors than a block has room for is not tried again.
+// (its error, if the staged pass meets it too, is that pass's to report).
 int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t limit,
                    std::vector<uint32_t>& settled, std::vector<uint32_t>& start) {
     const uint32_t k = g->terrains;
@@ -1541,10 +1561,13 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     const ResidentLayout lay(k, g->res_slots);
     unsigned char* d = g->d_resident;
     std::vector<ResidentCtrl> ctrl(k);
-    g->res_never.resize(k);
+    g->res_rest.resize(k);
+    const uint64_t slow_ns = resident_slow_ns(g);
     bool more = false;
     for (uint32_t t = 0; t < k; ++t) {
-        ctrl[t].done = g->res_never[t];
+        uint8_t& rest = g->res_rest[t];
+        ctrl[t].done = rest == kNeverResident || (rest && slow_ns);
+        if (rest && slow_ns && rest != kNeverResident) --rest;
         more |= !ctrl[t].done;
     }
     if (!more) return FL_OK;
@@ -1566,8 +1589,7 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     // a launch ends after some tens of milliseconds, so that other streams' solves run
     a.chunk = (uint32_t)std::max<uint64_t>(16, std::min<uint64_t>(1024, (1ull << 27) / std::max(1u, g->n)));
     a.limit = (uint32_t)limit;
-    // about what an iteration of the staged pass takes
-    a.slow_ns = k > 1 || fl::tuning().resident == 1 ? 0 : (400000ull + g->n) * (g->slope ? 2 : 1);
+    a.slow_ns = slow_ns;
     a.row = g->d_row;
     a.col = g->d_col;
     a.len = g->d_len;
@@ -1622,11 +1644,13 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
             c.need_rank = 0;
             if (c.error != 0) {
                 again[t] = 1;
-                if (c.error == kErrCapacity) g->res_never[t] = 1;
-            } else if (c.slow) {
+                g->res_rest[t] = c.error == kErrLate ? kRestSolves : kNeverResident;
+            } else if (c.left) {
                 start[t] = c.iters;
+                g->res_rest[t] = kRestSolves;
             } else if (c.done) {
                 settled[t] = c.iters;
+                if (c.slow > 1) g->res_rest[t] = kRestSolves;   // settled before the rule's end
             } else {
                 more = true;
                 continue;
