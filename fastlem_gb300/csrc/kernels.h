@@ -305,6 +305,15 @@ constexpr size_t kResidentSmem = 226 * 1024; // shared memory of a block, at mos
 constexpr uint32_t kResidentPart = 448;
 constexpr uint32_t kResidentMaxRow = 64;     // longest adjacency row taken
 constexpr uint32_t kSlowPoints = 4;
+constexpr uint32_t kResidentWords = 5;       // a terrain's barrier words and its start's verdict
+// A launch's time: its blocks hold their SMs all the while, and another stream's kernels wait.
+// Terrains stop after the iteration in which it is over and none starts after it; the next
+// launch goes on from there.
+// A 1,000-site solve of 20 iterations beside one of 250,007 sites with slope limits takes
+// 112 ms with unbounded launches, 29 with 10 ms, 8 with 3 ms (beside staged iterations
+// 9.7); the large one as long as ever.  A pack's launch starts with fewer terrains than fill
+// the SMs evenly: 48 terrains to convergence take 110 ms unbounded, 112 with 10 ms, 114 with 5.
+constexpr uint64_t kResidentShareNs = 3000000, kResidentSharePackNs = 10000000;
 // A terrain's device sites [lo, lo + n), cut into `parts` block ranges; slot0: its first
 // (terrain, part) slot.
 struct ResidentTerrain {
@@ -321,11 +330,12 @@ struct ResidentCtrl {
     uint32_t pad[2];
 };
 struct ResidentArgs {
-    uint32_t n, cap, slots, chunk;   // chunk: most iterations of a terrain per launch
+    uint32_t n, cap, slots;
     uint32_t limit;
     // an iteration over this counts one point and one over twice this kSlowPoints, one that
     // is not clears them, and kSlowPoints end the terrain's solve; 0: no rule
     uint64_t slow_ns;
+    uint64_t share_ns;
     bool rank_ready;
     const uint32_t *row, *col;
     const double* len;
@@ -343,8 +353,9 @@ struct ResidentArgs {
     const ResidentTerrain* terrains;
     const uint32_t* slot_terrain;
     ResidentCtrl* ctrl;
-    unsigned long long* bars;        // four per terrain, zero at launch
+    unsigned long long* bars;        // kResidentWords per terrain, zero at launch
     uint32_t* ticket;                // zero at launch
+    unsigned long long* started;     // when the launch's first block did (global_ns); zero at launch
 };
 size_t resident_smem(uint32_t cap, bool slope);
 uint32_t resident_cap(bool slope);   // most sites of a block

@@ -148,6 +148,11 @@ __device__ __forceinline__ unsigned long long& wait_until() {
     return ns;
 }
 constexpr unsigned long long kNoTime = ~0ull;
+// When the launch's share of time is over (shared).
+__device__ __forceinline__ unsigned long long& share_end() {
+    __shared__ unsigned long long ns;
+    return ns;
+}
 
 __device__ __forceinline__ bool give_up(Group& gr, uint32_t& spins) {
     if (++spins > kSpinLimit) {
@@ -547,10 +552,11 @@ __device__ __forceinline__ bool settle_down(const ResidentArgs& a, Group& gr, co
     return __syncthreads_or(lost) == 0;
 }
 
-// One terrain's iterations up to its fixed point, its limit or the launch's share.
+// One terrain's iterations up to its fixed point, its limit or the end of the launch's share.
 template <bool kSlope>
 __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, Group& gr) {
     __shared__ uint32_t s_fin, s_far, s_out, s_list;
+    __shared__ unsigned long long s_since;    // part 0: when the iteration started
     const uint32_t tid = threadIdx.x;
     const uint32_t each = tr.n / tr.parts, rest = tr.n % tr.parts;
     const uint32_t lo = tr.lo + gr.part * each + min(gr.part, rest);
@@ -559,7 +565,6 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
     ResidentCtrl* ctrl = gr.ctrl;
 
     uint32_t it = ctrl->iters;
-    const uint32_t stop = (uint32_t)min((uint64_t)it + a.chunk, (uint64_t)a.limit);
     bool valid = it > 0;                      // w, wa, wl hold the previous iteration's
 #pragma unroll 1
     for (uint32_t v = tid; v < S; v += kT) {
@@ -574,10 +579,11 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
     if (tid == 0) stsd(bk.rec(bk.none), -0.0);
     group_barrier(gr, false);
 
-    uint32_t slow = 0;                        // the time rule's points
-    while (gr.ok && it < stop) {
+    const bool keeps_time = gr.part == 0 && tid == 0;
+    uint32_t slow = keeps_time ? ctrl->slow : 0;   // the time rule's points
+    if (keeps_time) s_since = global_ns();
+    while (gr.ok) {
         const uint32_t par = it & 1u;
-        const uint64_t t0 = a.slow_ns && gr.part == 0 && tid == 0 ? global_ns() : 0;
         // ---- receivers
         bool lake = false;
         if (tid == 0) s_fin = s_far = s_out = s_list = 0;
@@ -886,22 +892,25 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
             }
         }
         ++it;
-        if (t0) {
-            const uint64_t took = global_ns() - t0;
-            slow = took <= a.slow_ns ? 0 : slow + (took > 2 * a.slow_ns ? kSlowPoints : 1);
+        bool ask = false;
+        if (keeps_time) {
+            const unsigned long long now = global_ns(), took = now - s_since;
+            if (a.slow_ns) slow = took <= a.slow_ns ? 0 : slow + (took > 2 * a.slow_ns ? kSlowPoints : 1);
+            ask = slow >= kSlowPoints || now > share_end();
+            s_since = now;
         }
-        const bool more = group_barrier(gr, changed, slow >= kSlowPoints);
+        const bool more = group_barrier(gr, changed, ask);
         if (!gr.ok) break;
         if (!more || it >= a.limit) {
-            if (gr.part == 0 && tid == 0) ctrl->done = 1;
+            if (keeps_time) ctrl->done = 1;
             break;
         }
         if (gr.stop) {                        // long rivers: the staged pass goes on
-            if (gr.part == 0 && tid == 0) ctrl->left = 1;
+            if (keeps_time) ctrl->left = slow >= kSlowPoints;
             break;
         }
     }
-    if (gr.part == 0 && tid == 0) {
+    if (keeps_time) {
         ctrl->iters = it;
         ctrl->slow = slow;
     }
@@ -910,6 +919,11 @@ __device__ void solve_terrain(const ResidentArgs& a, const ResidentTerrain& tr, 
 template <bool kSlope>
 __global__ void __launch_bounds__(kT, 1) k_resident(const __grid_constant__ ResidentArgs a) {
     __shared__ uint32_t s_slot;
+    __shared__ bool s_go;
+    if (threadIdx.x == 0) {
+        const unsigned long long now = global_ns(), first = atomicCAS(a.started, 0ull, now);
+        share_end() = (first ? first : now) + a.share_ns;
+    }
     while (true) {
         __syncthreads();
         if (threadIdx.x == 0) s_slot = atomicAdd(a.ticket, 1u);
@@ -918,8 +932,16 @@ __global__ void __launch_bounds__(kT, 1) k_resident(const __grid_constant__ Resi
         if (slot >= a.slots) return;
         const uint32_t t = a.slot_terrain[slot];
         const ResidentTerrain tr = a.terrains[t];
-        Group gr{a.bars + 4ull * t, a.ctrl + t, tr.parts, slot - tr.slot0, 0, true, false};
+        unsigned long long* const words = a.bars + (unsigned long long)kResidentWords * t;
+        Group gr{words, a.ctrl + t, tr.parts, slot - tr.slot0, 0, true, false};
         if (gr.ctrl->done) continue;          // settled in an earlier launch
+        // its first block decides for all of them whether there is time to start
+        if (threadIdx.x == 0) {
+            const unsigned long long mine = global_ns() > share_end() ? 2 : 1, first = atomicCAS(&words[4], 0ull, mine);
+            s_go = (first ? first : mine) == 1;
+        }
+        __syncthreads();
+        if (!s_go) continue;
         solve_terrain<kSlope>(a, tr, gr);
     }
 }

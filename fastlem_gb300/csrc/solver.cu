@@ -496,7 +496,7 @@ struct fl_graph {
     int stamp = 0;
     uint32_t last_meta[kMetaCount] = {};
     // whole solves in one launch (resident.cu): the terrains' parts, in one device block
-    // of ticket, barrier words (zeroed per launch), progress, terrains and slots
+    // of ticket, start and barrier words (zeroed per launch), progress, terrains and slots
     bool resident = false;
     bool simple = false;         // rows mutual, no site named twice (check_resident)
     bool res_slope = false;              // the plan has room for slope limits
@@ -1419,10 +1419,10 @@ int finish_generate(fl_graph* g, HostCols<double> out_elev, uint32_t iters, uint
 
 // Offsets in fl_graph::d_resident for k terrains.
 struct ResidentLayout {
-    uint64_t ticket = 0, bars, ctrl, terrains, slots, bytes;
+    uint64_t ticket = 0, started = 8, bars, ctrl, terrains, slots, bytes;
     ResidentLayout(uint32_t k, uint32_t n_slots) {
         bars = 64;
-        ctrl = bars + 32ull * k;
+        ctrl = bars + 8ull * kResidentWords * k;
         terrains = ctrl + sizeof(ResidentCtrl) * k;
         slots = terrains + sizeof(ResidentTerrain) * k;
         bytes = slots + 4ull * n_slots;
@@ -1586,10 +1586,9 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     a.n = g->n;
     a.cap = g->res_cap;
     a.slots = g->res_slots;
-    // a launch ends after some tens of milliseconds, so that other streams' solves run
-    a.chunk = (uint32_t)std::max<uint64_t>(16, std::min<uint64_t>(1024, (1ull << 27) / std::max(1u, g->n)));
     a.limit = (uint32_t)limit;
     a.slow_ns = slow_ns;
+    a.share_ns = k == 1 ? kResidentShareNs : kResidentSharePackNs;
     a.row = g->d_row;
     a.col = g->d_col;
     a.len = g->d_len;
@@ -1619,6 +1618,7 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     a.ctrl = reinterpret_cast<ResidentCtrl*>(d + lay.ctrl);
     a.bars = reinterpret_cast<unsigned long long*>(d + lay.bars);
     a.ticket = reinterpret_cast<uint32_t*>(d + lay.ticket);
+    a.started = reinterpret_cast<unsigned long long*>(d + lay.started);
     g->w_valid = false;
     std::vector<uint8_t> ended(k), again(k);
     for (uint32_t t = 0; t < k; ++t) ended[t] = ctrl[t].done != 0;

@@ -220,7 +220,7 @@ int fl_select_device(int device);
 int fl_graph_set_timing(fl_graph* g, int enable);
 void fl_graph_reset_stats(fl_graph* g);
 /* Blocking host synchronisations the model's calls made since the last reset: one per
- * staged iteration of generate() (one for all iterations of a resident solve), one more in
+ * staged iteration of generate(), one per launch of a resident solve, one more in
  * an iteration that computes the lake order. */
 uint64_t fl_graph_host_syncs(const fl_graph* g);
 
