@@ -205,7 +205,12 @@ __device__ __forceinline__ uint32_t steepest(const ResidentArgs& a, uint32_t g) 
         for (int k = 0; k < 4; ++k)
             if (b + k < s1) sc.consider(b + k, e[k], f[k]);
     }
-    return sc.decided() ? sc.slot : steepest_exact(a.row, a.col, a.len, a.elev, g);
+    if (sc.decided()) return sc.slot;
+    if (sc.close && !sc.exact) {
+        const uint32_t slot = steepest_bits(a.col, a.ilen, a.elev, g, s0, s1);
+        if (slot != kUndecided) return slot;
+    }
+    return steepest_exact(a.row, a.col, a.len, a.elev, g);
 }
 
 __device__ __forceinline__ double edge_or_one(const ResidentArgs& a, uint32_t i, uint32_t j) {
