@@ -63,6 +63,7 @@ constexpr uint64_t kPendingBits = 0x7ff4000000000000ull;
 // Rows up to this many slots are gathered with all loads in flight at once; longer
 // rows (rare: hull sites) take the plain loop.
 constexpr int kRowFast = 12;
+static_assert(kTileRow == kRowFast, "the rows that the tiles read");
 
 // The reference's drainage area of v given final donor areas: a_v + donors in
 // reverse adjacency order (generator.rs:154-159).  Column ids, then receivers,
@@ -150,9 +151,9 @@ __device__ __forceinline__ void scan_levels(uint32_t* s_cnt) {
 
 // Writes hgt (level of the inner sites, kNone of the outer ones), A of the inner sites, and
 // pending of the outer ones: the number of their outer donors (zeroed before; each donor
-// counts itself in).  Inner and settled sites have pending kNone.  Without `tiles` -- rows
-// that name a site twice or are not mutual, where a row does not tell its site's donors --
-// every site is an outer one.
+// counts itself in).  Inner and settled sites have pending kNone.  Without `tiles` -- short
+// rows that name a site twice or not at all although it names theirs, so that a row does not
+// tell its site's donors -- every site is an outer one.
 __global__ void __launch_bounds__(kTileThreads, kTileUpBlocks)
 k_tile_up(uint32_t n, const uint32_t* __restrict__ row, const uint32_t* __restrict__ col,
           const uint32_t* __restrict__ next, const double* __restrict__ area,

@@ -211,7 +211,7 @@ struct BasinArgs {
     uint32_t* tokslot;      // per donor-list entry: the slot whose list it is
     uint32_t* pend;         // per layout slot: chain bottoms still to push into its list
     uint32_t tok_cap;
-    bool tiles;             // the graph's rows are mutual and name no site twice
+    bool tiles;             // short rows name every site that names theirs, and once
     uint64_t* push_to;      // per site: (stamp << 32) | tokval index its chain bottom fills
     int* bu_done;
     int* td_need;
@@ -304,6 +304,7 @@ constexpr size_t kResidentSmem = 226 * 1024; // shared memory of a block, at mos
 // 87.4 / 170.
 constexpr uint32_t kResidentPart = 448;
 constexpr uint32_t kResidentMaxRow = 64;     // longest adjacency row taken
+constexpr uint32_t kTileRow = 12;            // longest row of a tile's inner site (basin.cu)
 constexpr uint32_t kSlowPoints = 4;
 constexpr uint32_t kResidentWords = 5;       // a terrain's barrier words and its start's verdict
 // A launch's time: its blocks hold their SMs all the while, and another stream's kernels wait.
@@ -361,9 +362,9 @@ size_t resident_smem(uint32_t cap, bool slope);
 uint32_t resident_cap(bool slope);   // most sites of a block
 uint32_t resident_blocks();          // most blocks of a launch
 cudaError_t launch_resident(const ResidentArgs& a, bool slope, uint32_t blocks, cudaStream_t st);
-// *bad = 1 unless the graph is simple (see resident.cu).
-void launch_check_simple(cudaStream_t st, uint32_t n, const uint32_t* row, const uint32_t* col,
-                         int* bad);
+// bad[0] = 1 unless the resident solve takes the graph, bad[1] = 1 unless the tiles do (see
+// resident.cu).
+void launch_check_rows(cudaStream_t st, uint32_t n, const uint32_t* row, const uint32_t* col, int* bad);
 
 // One drainage-area / response-time / elevation pass on final receivers.
 cudaError_t basin_pass(const BasinArgs& a, cudaStream_t st, const Hooks& hk, uint32_t nnz);

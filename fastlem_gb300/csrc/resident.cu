@@ -951,27 +951,50 @@ __global__ void __launch_bounds__(kT, 1) k_resident(const __grid_constant__ Resi
     }
 }
 
-// Whether every edge of the graph appears exactly once in either end's row, no site is its
-// own neighbour and no row is longer than the donor count can hold.
-__global__ void k_check_simple(uint32_t n, const uint32_t* __restrict__ row,
-                               const uint32_t* __restrict__ col, int* __restrict__ bad) {
+// What a row tells of its site's donors: bad[0] unless every edge of the graph appears exactly
+// once in either end's row, no site is its own neighbour and no row is longer than the donor
+// count can hold (the resident solve's graphs); bad[1] unless every site is named exactly once
+// in each short row (kTileRow) of a site that it names (the tiles', which leave longer rows to
+// the rounds).  Rows longer than kResidentMaxRow are taken by their block together.
+__global__ void __launch_bounds__(kThreads) k_check_rows(uint32_t n, const uint32_t* __restrict__ row,
+                                                         const uint32_t* __restrict__ col, int* __restrict__ bad) {
+    __shared__ uint32_t s_long[kThreads], s_count;
+    if (threadIdx.x == 0) s_count = 0;
+    __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool b = false;
+    bool odd = false, unlike = false;
+    // how often site v's row [r0, r1) names u
+    auto times = [&](uint32_t r0, uint32_t r1, uint32_t u) {
+        uint32_t c = 0;
+        for (uint32_t q = r0; q < r1; ++q) c += col[q] == u;
+        return c;
+    };
     if (i < n) {
         const uint32_t s0 = row[i], s1 = row[i + 1];
-        b = s1 - s0 > kResidentMaxRow;
-        for (uint32_t s = s0; s < s1 && !b; ++s) {
-            const uint32_t j = col[s];
-            b = j == i;
-            for (uint32_t q = s + 1; q < s1; ++q) b |= col[q] == j;
-            uint32_t back = 0;
-            const uint32_t r0 = row[j], r1 = row[j + 1];
-            if (r1 - r0 > kResidentMaxRow) b = true;
-            for (uint32_t q = r0; q < r1 && !b; ++q) back += col[q] == i;
-            b |= back != 1;
+        const bool is_long = s1 - s0 > kResidentMaxRow;
+        odd = is_long;
+        if (is_long) s_long[atomicAdd(&s_count, 1u)] = i;
+        for (uint32_t s = s0; s < s1 && !is_long && !unlike; ++s) {
+            const uint32_t j = col[s], r0 = row[j], r1 = row[j + 1];
+            if (j == i) unlike = true;
+            if (r1 - r0 > kResidentMaxRow) odd = true;
+            else if (times(r0, r1, i) != 1) {
+                odd = true;
+                unlike |= r1 - r0 <= kTileRow;
+            }
+            if (!odd) odd = times(s + 1, s1, j) != 0;
         }
     }
-    if (__syncthreads_or(b) && threadIdx.x == 0) *bad = 1;
+    __syncthreads();
+    for (uint32_t l = 0; l < s_count; ++l) {
+        const uint32_t v = s_long[l];
+        for (uint32_t s = row[v] + threadIdx.x; s < row[v + 1] && !unlike; s += blockDim.x) {
+            const uint32_t j = col[s], r0 = row[j], r1 = row[j + 1];
+            unlike |= r1 - r0 <= kTileRow && times(r0, r1, v) != 1;
+        }
+    }
+    if (__syncthreads_or(odd || unlike) && threadIdx.x == 0) bad[0] = 1;
+    if (__syncthreads_or(unlike) && threadIdx.x == 0) bad[1] = 1;
 }
 
 }  // namespace
@@ -1000,9 +1023,8 @@ cudaError_t launch_resident(const ResidentArgs& a, bool slope, uint32_t blocks, 
     return cudaLaunchCooperativeKernel(kern, dim3(blocks), dim3(kT), argv, sm, st);
 }
 
-void launch_check_simple(cudaStream_t st, uint32_t n, const uint32_t* row, const uint32_t* col,
-                         int* bad) {
-    k_check_simple<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(n, row, col, bad);
+void launch_check_rows(cudaStream_t st, uint32_t n, const uint32_t* row, const uint32_t* col, int* bad) {
+    k_check_rows<<<(n + kThreads - 1) / kThreads, kThreads, 0, st>>>(n, row, col, bad);
 }
 
 }  // namespace fl

@@ -498,7 +498,7 @@ struct fl_graph {
     // whole solves in one launch (resident.cu): the terrains' parts, in one device block
     // of ticket, start and barrier words (zeroed per launch), progress, terrains and slots
     bool resident = false;
-    bool simple = false;         // rows mutual, no site named twice (check_resident)
+    bool tiles = false;          // the tiles take the graph (check_rows)
     bool res_slope = false;              // the plan has room for slope limits
     uint32_t largest = 0;                // sites of the largest terrain
     uint32_t res_cap = 0, res_slots = 0, res_blocks = 0;
@@ -1322,7 +1322,7 @@ int enqueue_basin_pass(fl_graph* g, bool all_records = false) {
     a.tokslot = g->d_tokslot;
     a.pend = g->d_pend;
     a.tok_cap = g->tok_cap;
-    a.tiles = g->simple;
+    a.tiles = g->tiles;
     a.push_to = g->d_push;
     a.bu_done = g->d_bu_done;
     a.td_need = g->d_td_need;
@@ -1429,20 +1429,20 @@ struct ResidentLayout {
     }
 };
 
-// Whether every terrain's graph is one the tiles and the resident solve take (at set-up; the model's
-// buffers are ready).
-int check_resident(fl_graph* g) {
+// Whether every terrain's graph is one that the tiles and that the resident solve take (at
+// set-up; the model's buffers are ready).
+int check_rows(fl_graph* g) {
     for (uint32_t t = 0; t < g->terrains; ++t)
         g->largest = std::max(g->largest, g->site_off[t + 1] - g->site_off[t]);
     if (g->n >= 0x80000000u) return FL_OK;
-    FL_CU(cudaMemsetAsync(g->d_flags, 0, sizeof(int), g->stream));
-    fl::launch_check_simple(g->stream, g->n, g->d_row, g->d_col, g->d_flags);
+    FL_CU(cudaMemsetAsync(g->d_flags, 0, 2 * sizeof(int), g->stream));
+    fl::launch_check_rows(g->stream, g->n, g->d_row, g->d_col, g->d_flags);
     FL_CU(cudaGetLastError());
-    FL_CU(cudaMemcpyAsync(g->h_status, g->d_flags, sizeof(int), cudaMemcpyDeviceToHost, g->stream));
-    FL_CU(cudaMemsetAsync(g->d_flags, 0, sizeof(int), g->stream));
+    FL_CU(cudaMemcpyAsync(g->h_status, g->d_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost, g->stream));
+    FL_CU(cudaMemsetAsync(g->d_flags, 0, 2 * sizeof(int), g->stream));
     FL_CU(cudaStreamSynchronize(g->stream));
-    g->simple = g->h_status[0] == 0;
-    g->resident = g->simple && g->largest <= (uint64_t)fl::resident_blocks() * fl::resident_cap(false);
+    g->tiles = g->h_status[1] == 0;
+    g->resident = g->h_status[0] == 0 && g->largest <= (uint64_t)fl::resident_blocks() * fl::resident_cap(false);
     return FL_OK;
 }
 
@@ -1935,7 +1935,7 @@ int create_graph(uint32_t n, const uint32_t* row_ptr, const uint32_t* col, const
     }
     g->def_outlets.resize(n_default);
     for (uint32_t i = 0; i < n_default; ++i) g->def_outlets[i] = g->inv[default_outlets[i]];
-    if ((rc = check_resident(g))) return fail(rc);
+    if ((rc = check_rows(g))) return fail(rc);
     *out = g;
     return FL_OK;
 }
