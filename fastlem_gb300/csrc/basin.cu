@@ -1976,7 +1976,7 @@ cudaError_t basin_pass(const BasinArgs& a, cudaStream_t st, const Hooks& hk, uin
     k_tile_up<<<tiles, kTileThreads, 0, st>>>(n, a.row, a.col, a.next, a.area, a.A, a.pending, a.hgt,
                                               a.tid, titer, a.tiles);
     k_collect_front<<<g_compact, kRoundBlock, 0, st>>>(n, a.pending, a.order, a.meta + kMetaLeaves);
-    hk.end(hk.ctx, kcBasinBuild, 20.0 * n);
+    hk.end(hk.ctx, kcBasinBuild, 40.0 * n + 4.0 * nnz);
 
     // Kahn rounds: order 4 + next 4 + row 8 + area 8 + A 8 + hgt 4 + pending 4 per site,
     // col 4 + next 4 per slot, donor areas 8 per site
@@ -1984,7 +1984,7 @@ cudaError_t basin_pass(const BasinArgs& a, cudaStream_t st, const Hooks& hk, uin
     e = coop_launch(k_kahn, g_kahn, kThreads, st, n, a.row, a.col, a.next, a.area, a.A, a.pending,
                     a.hgt, a.order, a.roff, a.rtime, a.max_rounds, a.kahn_min_width, a.meta,
                     a.flags);
-    hk.end(hk.ctx, kcKahn, 48.0 * n + 8.0 * nnz);
+    hk.end(hk.ctx, kcKahn, 0.0);
     if (e != cudaSuccess) return e;
 
     hk.begin(hk.ctx);
@@ -2099,7 +2099,7 @@ cudaError_t basin_pass(const BasinArgs& a, cudaStream_t st, const Hooks& hk, uin
         tile_down<<<tiles, kTileThreads, smem, st>>>(n, td, a.hgt, a.all_records);
         e = cudaGetLastError();
     }
-    hk.end(hk.ctx, kcLowDown, 112.0 * n);
+    hk.end(hk.ctx, kcLowDown, 16.0 * n);
     return e;
 }
 

@@ -317,6 +317,17 @@ __global__ void k_rec_times(uint32_t n, const fl::TRec* __restrict__ rec, double
     if (i < n) t[i] = rec[i].t;
 }
 
+// Marks the sites that another one drains to, and counts the others (statistics).
+__global__ void k_mark_receivers(uint32_t n, const uint32_t* __restrict__ next, uint32_t* __restrict__ mark) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && next[i] != i) mark[next[i]] = 1;
+}
+__global__ void k_count_unmarked(uint32_t n, const uint32_t* __restrict__ mark, uint32_t* __restrict__ count) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int c = __syncthreads_count(i < n && mark[i] == 0);
+    if (threadIdx.x == 0 && c) atomicAdd(count, (uint32_t)c);
+}
+
 __global__ void k_fill_f64(uint32_t n, double* __restrict__ a, const double* __restrict__ src) {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) a[i] = src ? src[i] : 0.0;
@@ -501,6 +512,7 @@ struct fl_graph {
     bool tiles = false;          // the tiles take the graph (check_rows)
     bool res_slope = false;              // the plan has room for slope limits
     uint32_t largest = 0;                // sites of the largest terrain
+    bool solved = false;                 // d_next holds a pass's receivers
     uint32_t res_cap = 0, res_slots = 0, res_blocks = 0;
     unsigned char* d_resident = nullptr;
     // per terrain: solves under the time rule that it sits out, kNeverResident: all solves
@@ -1217,8 +1229,13 @@ int enqueue_lakes(fl_graph* g, const int* gate, bool reroute) {
 }
 
 // Drainage areas, response times, elevations on final receivers; *changed.
-// Algorithmic bytes of the kernels that work on the skeleton, whose size is known
-// only once the pass has run (the launch groups were counted with 0 bytes).
+// Algorithmic bytes of the kernels that work on the rounds' and the tiles' sites and on the
+// skeleton, whose numbers are known only once the pass has run (the launch groups were counted
+// with 0 bytes, or with what every site takes).
+//   rounds up: order, next (8), row (8), area and A (16), hgt (4), pending atomic (4) in and
+//              out (4), round order (4) per site, column and receiver (8) per slot
+//   rounds down: receiver's record (32), w, inputs and elevation (48), own record (32)
+//   tiles down: uplift, elevation in and out (24) [+ tangent, distance (16)] per inner site
 //   bottom-up: slot record (32) + slot info (8) + area out (8) per slot;
 //              offset, length, bottom id, bottom area, hand-off flag (24) per chain
 //   top-down:  w (8) + flags (1) + t out (8) [+ elevation out (8) with slope limits]
@@ -1227,7 +1244,12 @@ int enqueue_lakes(fl_graph* g, const int* gate, bool reroute) {
 //   ranking:   per pointer-jumping round, own and successor's pointer and distance
 //              in (16) and out (8) per skeleton site; ceil(log2(longest chain)) + 1
 //              rounds
-void account_skeleton(fl_graph* g) {
+void account_pass(fl_graph* g) {
+    const double rounds_n = g->last_meta[kMetaFrontBeg];
+    g->k_bytes[kcKahn] += (48.0 + 8.0 * g->nnz / g->n) * rounds_n;
+    g->k_bytes[kcLowDown] += 112.0 * rounds_n;
+    if (g->tiles)
+        g->k_bytes[kcLowDown] += (g->slope ? 40.0 : 24.0) * (g->n - rounds_n - g->last_meta[kMetaNs]);
     const double ns = g->last_meta[kMetaNs], nc = g->last_meta[kMetaChains];
     const uint32_t longest = g->last_meta[kMetaMaxChain];
     int rounds = 1;
@@ -1241,6 +1263,7 @@ void account_skeleton(fl_graph* g) {
 // hold its outcome once it has run (finish_basin_pass).  all_records: every site's
 // top-down record is read afterwards (response times).
 int enqueue_basin_pass(fl_graph* g, bool all_records = false) {
+    g->solved = true;
     g->stamp = g->stamp == 0x7ffffff0 ? 1 : g->stamp + 1;
     if (g->stamp == 1) {   // stamps wrapped (or first pass): clear hand-off words
         FL_CU(cudaMemsetAsync(g->d_bu_done, 0, g->n * 4ull, g->stream));
@@ -1344,7 +1367,7 @@ int enqueue_basin_pass(fl_graph* g, bool all_records = false) {
 int finish_basin_pass(fl_graph* g, const int* h) {
     FL_TRY(device_error(h));
     g->w_valid = true;
-    account_skeleton(g);
+    account_pass(g);
     return FL_OK;
 }
 
@@ -1587,6 +1610,7 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     a.cap = g->res_cap;
     a.slots = g->res_slots;
     a.limit = (uint32_t)limit;
+    g->solved = true;
     a.slow_ns = slow_ns;
     a.share_ns = k == 1 ? kResidentShareNs : kResidentSharePackNs;
     a.row = g->d_row;
@@ -1620,7 +1644,9 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
     a.ticket = reinterpret_cast<uint32_t*>(d + lay.ticket);
     a.started = reinterpret_cast<unsigned long long*>(d + lay.started);
     g->w_valid = false;
+    std::memset(g->last_meta, 0, sizeof g->last_meta);   // of no staged pass any more
     std::vector<uint8_t> ended(k), again(k);
+    std::vector<uint32_t> counted(k, 0);
     for (uint32_t t = 0; t < k; ++t) ended[t] = ctrl[t].done != 0;
     while (more) {
         FL_CU(cudaMemsetAsync(d, 0, lay.ctrl, g->stream));
@@ -1640,6 +1666,13 @@ int resident_solve(fl_graph* g, const std::vector<uint32_t>& outlets, uint64_t l
         for (uint32_t t = 0; t < k; ++t) {
             ResidentCtrl& c = ctrl[t];
             if (ended[t]) continue;
+            // an iteration's algorithmic bytes: row (8), own and new pair (16), area (8),
+            // receiver and distance out (12), links' row (8), w's operands and w (32), uplift,
+            // outlet flag, elevation in and out (25) [+ tangent and distance (24)] per site;
+            // columns twice, 1/len and neighbour's pair (20) per slot
+            g->k_bytes[kcResident] += (c.iters - counted[t]) * (double)(g->site_off[t + 1] - g->site_off[t]) *
+                                      (109.0 + (g->slope ? 24.0 : 0.0) + 20.0 * g->nnz / g->n);
+            counted[t] = c.iters;
             need_rank |= c.need_rank != 0;
             c.need_rank = 0;
             if (c.error != 0) {
@@ -2327,7 +2360,18 @@ int fl_graph_basin_stats(const fl_graph* g, uint64_t* out, uint32_t cap) {
     const uint32_t* m = g->last_meta;
     auto u64 = [&](int slot) { return (uint64_t)m[slot] | ((uint64_t)m[slot + 1] << 32); };
     const uint64_t up = u64(kMetaUpSlow), down = u64(kMetaDownSlow);
-    const uint64_t vals[] = {m[kMetaRStop], m[kMetaLeaves], m[kMetaNs], m[kMetaChains],
+    uint32_t leaves = 0;
+    if (g->solved && cap > 1) {              // from the last pass's receivers
+        FL_CU(cudaSetDevice(g->device));
+        FL_CU(cudaMemsetAsync(g->d_pending, 0, g->n * 4ull, g->stream));
+        FL_CU(cudaMemsetAsync(g->d_meta, 0, 4, g->stream));
+        k_mark_receivers<<<blocks_for(g->n), kThreads, 0, g->stream>>>(g->n, g->d_next, g->d_pending);
+        k_count_unmarked<<<blocks_for(g->n), kThreads, 0, g->stream>>>(g->n, g->d_pending, g->d_meta);
+        FL_CU(cudaGetLastError());
+        FL_CU(cudaMemcpyAsync(&leaves, g->d_meta, 4, cudaMemcpyDeviceToHost, g->stream));
+        FL_CU(cudaStreamSynchronize(g->stream));
+    }
+    const uint64_t vals[] = {m[kMetaRStop], leaves, m[kMetaNs], m[kMetaChains],
                              m[kMetaMaxChain], m[kMetaSlow], m[kMetaSpinUp], m[kMetaSpinDown],
                              (up >> kStatDurShift) << 6, ((up >> kStatCycShift) & kStat22) << 7,
                              up & kStat20,

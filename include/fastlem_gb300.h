@@ -261,15 +261,17 @@ uint32_t fl_num_kernel_classes(void);
 int fl_graph_kernel_stats(const fl_graph* g, uint32_t cls, const char** name, uint64_t* launches,
                           double* device_ms, double* bytes);
 
-/* Shape of the last staged basin pass (up to `cap` values; a resident solve leaves them as
- * they were): Kahn rounds run, sites of the first round, skeleton sites, skeleton chains, longest chain, skeleton sites needing the full
+/* Shape of the last basin pass (up to `cap` values; after a resident solve all but the leaves
+ * are zero): Kahn rounds run, leaves (counted on the device by this call, from the pass's
+ * receivers), skeleton sites, skeleton chains, longest chain, skeleton sites needing the full
  * pull while walking, bottom-up and top-down hand-off wait iterations; then the
  * slowest bottom-up chain's walk time (ns), SM cycles spent in its full pulls and
  * their number; the slowest top-down chain's walk time (ns), SM cycles waiting for
  * its parent and its length.  Durations are kept to 64 ns, cycles to 128. */
 int fl_graph_basin_stats(const fl_graph* g, uint64_t* out, uint32_t cap);
 
-/* Round structure of the last staged basin pass (instrumentation; no fastlem counterpart).
+/* Round structure of the last basin pass (instrumentation; no fastlem counterpart; a resident
+ * solve has no rounds).
  * *rounds = Kahn rounds run (r); for k <= min(cap - 1, r): offsets[k] = first order
  * slot of Kahn round k, up_ns[k] = device clock (ns) when bottom-up round k started
  * (up_ns[r] = end), down_ns[k] = when the k-th top-down round started (highest Kahn
