@@ -13,7 +13,6 @@ constexpr int kThreads = 256;
 enum Flag {
     kHasLake = 0,   // some non-outlet site has no lower neighbour
     kChanged = 1,   // some elevation changed this iteration
-    kJumped = 2,    // a pointer-jumping round changed something
     kError = 3,     // device-side limit hit (see kErr* codes)
     kBarrier = 4,   // grid barrier arrival counter
     kBarrierGen = 5,// grid barrier generation

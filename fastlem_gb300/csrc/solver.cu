@@ -188,11 +188,6 @@ __device__ __forceinline__ double edge_len_or_one(const uint32_t* __restrict__ r
     return 1.0;
 }
 
-__global__ void k_copy_u32(uint32_t n, const uint32_t* __restrict__ a, uint32_t* __restrict__ b) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) b[i] = a[i];
-}
-
 struct LakeArgs {
     uint32_t n;
     const uint32_t *row, *col;
@@ -477,7 +472,7 @@ struct fl_graph {
     // from, for the current parameters (cleared whenever d_w is reused or k uploaded)
     bool w_valid = false;
     uint32_t *d_next = nullptr, *d_lab = nullptr, *d_lab2 = nullptr, *d_rank = nullptr,
-             *d_sor = nullptr, *d_outlets = nullptr, *d_bas = nullptr;
+             *d_sor = nullptr, *d_outlets = nullptr;
     uint8_t* d_outlet = nullptr;
     unsigned long long* d_best = nullptr;
     int* d_flags = nullptr;
@@ -590,7 +585,7 @@ void free_graph(fl_graph* g) {
     if (!g) return;
     void* ptrs[] = {g->d_row, g->d_col, g->d_len, g->d_area, g->d_k, g->d_u, g->d_tan, g->d_base,
                     g->d_elev, g->d_A, g->d_t, g->d_w, g->d_rlen, g->d_next, g->d_lab, g->d_lab2,
-                    g->d_rank, g->d_sor, g->d_outlets, g->d_bas, g->d_outlet, g->d_best,
+                    g->d_rank, g->d_sor, g->d_outlets, g->d_outlet, g->d_best,
                     g->d_flags, g->d_pending, g->d_hgt, g->d_order, g->d_roff, g->d_meta,
                     g->d_sid, g->d_slist, g->d_desig, g->d_sptr0, g->d_sdist0, g->d_sptr1,
                     g->d_sdist1, g->d_cid, g->d_cbot, g->d_clen, g->d_coff, g->d_layout,
@@ -690,7 +685,6 @@ int alloc_workspace(fl_graph* g) {
     FL_TRY(dalloc(&g->d_rank, n));
     FL_TRY(dalloc(&g->d_sor, n));
     FL_TRY(dalloc(&g->d_outlets, n));
-    FL_TRY(dalloc(&g->d_bas, n));
     FL_TRY(dalloc(&g->d_trec, n));
     FL_TRY(dalloc(&g->d_outlet, n));
     FL_TRY(dalloc(&g->d_best, n));
