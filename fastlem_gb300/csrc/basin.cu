@@ -121,7 +121,7 @@ __device__ __forceinline__ bool settled(const uint32_t* tid, const uint32_t* tit
 // than four donors makes its site an outer one.
 //
 // Both kernels are chains of shared-memory steps between block barriers, bound by their
-// latency (no pipe above 35 %, DRAM below 10 %), so three blocks share an SM.  Per iteration
+// latency (no pipe above 35 %, DRAM below 15 %), so three blocks share an SM.  Per iteration
 // at 16M / 1M sites: the rounds alone took 1,145 / 264 us up (21 / 20 of them) and 890 / 141 us
 // down; behind the tiles they take 296 / 152 us (14 / 13) and 167 / 69 us, the tiles 610 / 80 us
 // up and 605 / 52 us down, and the donor count over all sites is gone (100 us at 16M).  With

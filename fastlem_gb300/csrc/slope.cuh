@@ -26,8 +26,9 @@ __device__ __forceinline__ float2 float_pair(double e) {
 // The steepest of a row's slots by estimate.  With d = e_i - e_j, its estimate
 // (hi_i - hi_j) + (lo_i - lo_j) is within 2^-23 |d| + 2^-45.4 |e_i| of it (two roundings of
 // 2^-24; the pairs' errors and the rounding of lo_i - lo_j), so beyond 2^-24 |e_i| it has
-// d's sign and a relative error below 2^-21.  The slope estimate adds the slot's 1/len and
-// a product (2^-24 each): below 2^-20, as receivers.cu's comparison margin of 2^-17 needs.
+// d's sign and a relative error below 2^-21.4 + 2^-23 < 2^-20.9.  The slope estimate adds the
+// slot's 1/len and a product (2^-24 each): below 2^-20.6, well within receivers.cu's comparison
+// margin of 2^-17.
 // Rows with a difference below that threshold (or NaN) are scanned from the doubles' bits
 // (steepest_bits); slopes out of range and near-ties are left to the f64 scan.
 struct PairScan {

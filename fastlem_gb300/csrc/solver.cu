@@ -384,7 +384,7 @@ Tuning& tuning() {
 // fastlem_gb300/autotune.py); a CPU test keeps the two equal.
 const std::vector<ScheduleEntry>& schedule() {
     static const std::vector<ScheduleEntry> s = {
-        // max_sites, packed, {low_ilp, walk_per_sm, kahn_min_width}
+        // max_sites, packed, {low_ilp, walk_per_sm, kahn_min_width, sized_grids}
         {0x20000u, false, {4, 0, 0, false}},
         {0x80000u, false, {4, 0, 4096, false}},
         {0x200000u, false, {4, 0, 4096, true}},
@@ -1505,16 +1505,24 @@ int plan_resident(fl_graph* g) {
 // The largest terrain that the resident solve takes by default.  Its walks go site by site
 // (about 0.3 us a site of the longest river and direction), the staged pass folds whole
 // chains but pays some 400 us of launches, barriers and skeleton building an iteration.
-// Measured without slope limits (32 iterations, staged / resident, ms): 10,000 sites 10.6 /
-// 2.3, 150,000 16.5 / 11.6, 200,000 17.2 / 13.7, 230,000 17.4 / 17.2, 262,000 17.7 / 14.9,
-// 400,000 20.3 / 16.5, 450,000 25.5 / 36.3, 600,000 25.7 / 35.3 (the last two and the first before
-// the tiles).  With slope limits the staged walk is site by site too: 100,000 29.5 / 10.5,
-// 600,000 102 / 53.
+// Without slope limits, us an iteration, staged / resident, over four random terrains (three
+// from 330,000): of the first 32 iterations, in which rivers wander (the resident side's spread
+// is theirs), and of the first 128:
+//   65,537    378-396 / 157-195   356-375 / 130-151
+//   150,000   436-444 / 325-403   406-409 / 248-287
+//   200,000   459-494 / 350-486   422-431 / 274-321
+//   262,144   472-499 / 454-589   435-445 / 343-414
+//   330,000   502-518 / 426-604   464-472 / 375-436
+//   400,000   539-604 / 537-859   500-514 / 443-589
+//   500,000   554-617 / 607-854   518-535 / 540-591
+//   1,000,000 786-848 / 1,085-1,686   728-748 / 891-1,087
+// so the line lies where the early iterations break even.  With slope limits the staged walk is
+// site by site too: 100,000 sites 29.5 / 10.5 ms for 32 iterations, 600,000 102 / 53.
 constexpr uint32_t kResidentLargest = 262144, kResidentLargestSlope = 786432;
 // The most sites of all packed terrains together: a packed resident solve is bound by the
 // blocks' throughput, the staged one by its launches first.  Terrains of 47,000 sites, staged /
-// resident, ms an iteration: 1.5M sites 0.77 / 0.71, 3.0M 1.09 / 1.10, 4.5M 1.41 / 1.51, 9M 2.30 /
-// 2.89; with slope limits 3.0M 2.19 / 1.72, 4.5M 2.64 / 2.49, 6M 3.15 / 3.27.
+// resident, ms an iteration: 1.5M sites 0.78 / 0.70, 3.0M 1.11 / 1.13, 4.5M 1.38 / 1.55, 9M 2.29 /
+// 2.97; with slope limits 3.0M 2.19 / 1.78, 4.5M 2.61 / 2.60, 6M 3.08 / 3.42.
 constexpr uint64_t kResidentTotal = 3145728, kResidentTotalSlope = 5242880;
 
 // Whether generate() takes the resident solve: a tuning override of the staged pass's

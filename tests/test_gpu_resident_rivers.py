@@ -100,3 +100,22 @@ def test_file_in_a_pack(orc):
         seen = now
         for t, ((e, it), o) in enumerate(zip(want, outs)):
             assert int(g.last_terrain_iterations[t]) == it and _same(np.array(o.elevations()), e), t
+
+
+@pytest.mark.parametrize("iters", [3, 7, 40])
+def test_pack_leaves_at_different_iterations(orc, iters):
+    """The staged iterations count on from each terrain's own: one that left after some, one
+    that starts again, settled ones, and limits before and after they leave."""
+    ms = [workloads.build_model(9000, 95.0, 1, 0), _terrain_with_file(9000, 2900, 3), _file(30000),
+          _terrain_with_file(2500, 5000, 4), _file(40)]
+    ps = [_params(m) for m in ms]
+    want = [_oracle(orc, m, p, iters) for m, p in zip(ms, ps)]
+    batch = TerrainBatch(ms)
+    for call in range(2):
+        g = BatchGenerator().set_batch(batch).set_parameters(ps).set_max_iteration(iters)
+        outs = g.generate()
+        for t, ((e, it), o) in enumerate(zip(want, outs)):
+            assert int(g.last_terrain_iterations[t]) == it and _same(np.array(o.elevations()), e), t
+        assert g.last_iterations == max(it for _, it in want)
+    now = _launches(batch.handle())
+    assert now[0] > 0 and now[1] > 0
