@@ -53,7 +53,7 @@ struct Tuning {
     int64_t kahn_min_width = -1;
     int sized_grids = -1;
     bool gpu_rank = true;
-    int resident = -1;     // whole solves in one launch: 0 never
+    int resident = -1;     // many iterations a launch: 0 never
 };
 Tuning& tuning();
 // The shapes for a model of n sites (packed: several terrains), overrides applied.
@@ -296,7 +296,7 @@ RankResult gpu_lake_rank(cudaStream_t st, uint32_t n, const uint32_t* row, const
 // Runs the exact parallel fold over one chain of n operands starting at x0 (probe).
 cudaError_t fold_probe(const double* y, uint32_t n, double x0, double* out);
 
-// ---- whole solves in one launch (resident.cu) ----
+// ---- many iterations a launch (resident.cu) ----
 constexpr uint32_t kResidentEdges = 512;     // donors a block may have in other blocks
 constexpr size_t kResidentSmem = 226 * 1024; // shared memory of a block, at most
 // Sites of a block while there are blocks left.  us an iteration at 1,000 / 10,000 / 65,537

@@ -1,5 +1,5 @@
-// resident.cu -- whole solves in one kernel launch, for terrains whose working state fits
-// the SMs' shared memory (src/lem/generator.rs:140-210, every iteration, bit-exact).
+// resident.cu -- solves of many iterations a kernel launch, for terrains whose working state
+// fits the SMs' shared memory (src/lem/generator.rs:140-210, every iteration, bit-exact).
 //
 // The stage-by-stage pass (receivers.cu, solver.cu, basin.cu) spends an iteration of a
 // small or middling terrain on launches and grid barriers: about 28 dependent launches and
@@ -40,7 +40,9 @@
 // One launch takes many terrains (packed models): blocks take (terrain, part) slots in
 // order, largest terrains first, and a terrain starts when its last part is taken.  Only
 // the newest terrain can be partly taken, so the blocks that wait for its other parts wait
-// for terrains that are running.
+// for terrains that are running.  A launch ends by the clock (kResidentShareNs), and what a
+// terrain cannot finish here -- long rivers, too many far donors -- the staged pass takes over
+// (resident_solve in solver.cu).
 
 #include <algorithm>
 

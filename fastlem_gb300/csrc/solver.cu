@@ -501,7 +501,7 @@ struct fl_graph {
     uint32_t passes = 0;   // basin passes since the drainage areas were reset
     int stamp = 0;
     uint32_t last_meta[kMetaCount] = {};
-    // whole solves in one launch (resident.cu): the terrains' parts, in one device block
+    // many iterations a launch (resident.cu): the terrains' parts, in one device block
     // of ticket, start and barrier words (zeroed per launch), progress, terrains and slots
     bool resident = false;
     bool tiles = false;          // the tiles take the graph (check_rows)
@@ -1432,7 +1432,7 @@ int finish_generate(fl_graph* g, HostCols<double> out_elev, uint32_t iters, uint
     return FL_OK;
 }
 
-// ---- whole solves in one launch (resident.cu) ----
+// ---- many iterations a launch (resident.cu) ----
 
 // Offsets in fl_graph::d_resident for k terrains.
 struct ResidentLayout {

@@ -238,9 +238,10 @@ uint64_t fl_graph_host_syncs(const fl_graph* g);
  *                    rest of the GPU to other streams' solves), 0: whole-GPU grids
  *   "gpu_rank"       1: the lake heap's order computed on the GPU where lengths decide it
  *                    (the host heap otherwise), 0: always the host heap
- *   "resident"       whole solves in one launch: -1 for terrains up to the size where the
- *                    staged launches become faster, 1 for all that fit the SMs' shared
- *                    memory, 0 never (nor while one of the four shapes above is overridden)
+ *   "resident"       the resident solve (many iterations a launch): -1 for terrains up to the
+ *                    size where the staged launches become faster, while their rivers are not
+ *                    long, 1 for all that fit the SMs' shared memory, 0 never (nor while one of
+ *                    the four shapes above is overridden)
  * Change them only while no solve runs.  FL_LOW_ILP, FL_WALK_PER_SM, FL_KAHN_MIN_WIDTH,
  * FL_SIZED_GRIDS, FL_GPU_RANK and FL_RESIDENT in the environment set them at load. */
 int fl_set_tuning(const char* name, int64_t value);
